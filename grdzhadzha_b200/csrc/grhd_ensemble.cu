@@ -354,6 +354,8 @@ int build(grhd_ensemble *e)
         d.sb.cs = d.b.gvol();
         d.bg = host::background_of(hm.params, 0.0);
         d.o = host::options_of(hm.params);
+        d.fo64 = make_face_opt<double>(d.o);
+        d.fo32 = make_face_opt<float>(d.o);
         for (int q = 0; q < 3; ++q)
             d.inv[q] = hm.inverse_dx[q];
         d.cfl = hm.cfl;

@@ -655,7 +655,7 @@ template <typename T, bool MDOT, bool CG = false, int BGK = -1>
 __device__ __forceinline__ void
 faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
            T *__restrict__ rhs, const BoxDev &b, const Background &bg,
-           const Options &o, double idx0_, double idx1_, double idx2_,
+           const Options &o, const FaceOpt<T> &fo, double idx0_, double idx1_, double idx2_,
            int zchunk, int bx, int by, int bz, unsigned char *smem_raw,
            double *__restrict__ mdot_part, int64_t part)
 {
@@ -720,7 +720,7 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
             const int row = (bb + 2) * kPW;
             GeoT<T> gf;
             geo_avg_smem(Gc, nG, (bb + 1) * kGW + a, (bb + 1) * kGW + a + 1, gf);
-            const ConsT<T> f = face_flux(o, load_pv_smem(P, row + a),
+            const ConsT<T> f = face_flux(fo, load_pv_smem(P, row + a),
                                          load_pv_smem(P, row + a + 1),
                                          load_pv_smem(P, row + a + 2),
                                          load_pv_smem(P, row + a + 3), gf, 0);
@@ -739,7 +739,7 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
             GeoT<T> gf;
             geo_avg_smem(Gc, nG, bb * kGW + a + 1, (bb + 1) * kGW + a + 1, gf);
             const int col = a + 2;
-            const ConsT<T> f = face_flux(o, load_pv_smem(P, bb * kPW + col),
+            const ConsT<T> f = face_flux(fo, load_pv_smem(P, bb * kPW + col),
                                          load_pv_smem(P, (bb + 1) * kPW + col),
                                          load_pv_smem(P, (bb + 2) * kPW + col),
                                          load_pv_smem(P, (bb + 3) * kPW + col),
@@ -762,7 +762,7 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
             geo_load(Gc, nG, cell, gA);
             geo_load(Gn, nG, cell, gB);
             average_geo(gA, gB, gf);
-            Fhi = face_flux(o, w0, w1, w2, w3, gf, 2);
+            Fhi = face_flux(fo, w0, w1, w2, w3, gf, 2);
             // a box counts the sphere faces whose upper cell it holds, in
             // every direction, so the boxes of a level count each once
             if (MDOT && (cells ? k < b.hi[2] : k0 == b.lo[2]))
@@ -818,11 +818,11 @@ template <typename T, bool MDOT, int BGK>
 __global__ void __launch_bounds__(kTB *kTB, kMinBlocks<T>)
     k_faces(const T *__restrict__ prim, const T *__restrict__ src,
             T *__restrict__ rhs, BoxDev b, Background bg, Options o,
-            double idx0_, double idx1_, double idx2_, int zchunk,
-            double *__restrict__ mdot_part)
+            FaceOpt<T> fo, double idx0_, double idx1_, double idx2_,
+            int zchunk, double *__restrict__ mdot_part)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    faces_tile<T, MDOT, false, BGK>(prim, src, rhs, b, bg, o, idx0_, idx1_,
+    faces_tile<T, MDOT, false, BGK>(prim, src, rhs, b, bg, o, fo, idx0_, idx1_,
                                     idx2_, zchunk,
                         blockIdx.x, blockIdx.y, blockIdx.z, smem_raw,
                         mdot_part,
@@ -1518,6 +1518,16 @@ __device__ __forceinline__ double ens_dt(const EnsMember &m,
     return dt;
 }
 
+template <typename T>
+__device__ __forceinline__ const FaceOpt<T> &
+member_face_opt(const EnsMember &m)
+{
+    if constexpr (sizeof(T) == sizeof(double))
+        return m.fo64;
+    else
+        return m.fo32;
+}
+
 // The persistent ensemble kernel: `steps` RK4 steps of every member.
 // Phase 0: the CFL speed (when need_cfl), interior con2prim + sources and
 // the ghost fill of every state.  Each stage: ghost fill of the stage input
@@ -1664,18 +1674,19 @@ __global__ void __launch_bounds__(kEnsItemCells, kMinBlocks<T>)
                 const int64_t r = local / ms.tiles[0];
                 const int by = (int)(r % ms.tiles[1]);
                 const int bz = (int)(r / ms.tiles[1]);
+                const FaceOpt<T> &fo = member_face_opt<T>(ms);
                 if (ms.has_mdot)
                     faces_tile<T, true, true>(
                         static_cast<const T *>(ms.prim),
                         static_cast<const T *>(ms.src), static_cast<T *>(ms.k),
-                        ms.b, ms.bg, ms.o, ms.inv[0], ms.inv[1], ms.inv[2],
-                        a.zchunk, bx, by, bz, smem_raw, ms.mdot_part, local);
+                        ms.b, ms.bg, ms.o, fo, ms.inv[0], ms.inv[1],
+                        ms.inv[2], a.zchunk, bx, by, bz, smem_raw, ms.mdot_part, local);
                 else
                     faces_tile<T, false, true>(
                         static_cast<const T *>(ms.prim),
                         static_cast<const T *>(ms.src), static_cast<T *>(ms.k),
-                        ms.b, ms.bg, ms.o, ms.inv[0], ms.inv[1], ms.inv[2],
-                        a.zchunk, bx, by, bz, smem_raw, nullptr, local);
+                        ms.b, ms.bg, ms.o, fo, ms.inv[0], ms.inv[1],
+                        ms.inv[2], a.zchunk, bx, by, bz, smem_raw, nullptr, local);
             }
             if (!ens_barrier(a, ph++))
                 return;
@@ -1939,6 +1950,7 @@ __device__ __forceinline__ double log_sqrt_det6(const double *g)
 // source atmosphere, make_metric_source_derivative_stencil, :283-322).
 __global__ void __launch_bounds__(256, 2)
     k_ccz4_rhs(const double *__restrict__ s, BoxDev b, Options o,
+               FaceOpt<double> fo,
                const double *__restrict__ prim, const double *__restrict__ gc,
                double *__restrict__ rhs, int64_t rcs, double inv0,
                double inv1, double inv2, DevStatus *st)
@@ -1966,7 +1978,7 @@ __global__ void __launch_bounds__(256, 2)
                 const int64_t L = g - so + side * so, R = L + so;
                 Geo gf;
                 average_geo(geo_get(gc, n, L), geo_get(gc, n, R), gf);
-                f[side] = face_flux(o, load_pv_global<double>(prim, n, L - so),
+                f[side] = face_flux(fo, load_pv_global<double>(prim, n, L - so),
                                     load_pv_global<double>(prim, n, L),
                                     load_pv_global<double>(prim, n, R),
                                     load_pv_global<double>(prim, n, R + so),
@@ -2378,8 +2390,8 @@ void launch_faces(const T *prim, const T *src, T *rhs, const BoxDev &b,
     const bool md = o.accretion_radius > 0.0 && mdot_part;
     auto go = [&](auto kern) {
         kern<<<grid, block, faces_smem<T>(), s>>>(
-            prim, src, rhs, b, bg, o, inv_dx[0], inv_dx[1], inv_dx[2], zchunk,
-            md ? mdot_part : nullptr);
+            prim, src, rhs, b, bg, o, make_face_opt<T>(o), inv_dx[0],
+            inv_dx[1], inv_dx[2], zchunk, md ? mdot_part : nullptr);
     };
     if (bg.kind == 1)
         md ? go(k_faces<T, true, 1>) : go(k_faces<T, false, 1>);
@@ -2509,7 +2521,8 @@ void launch_ccz4_rhs(const double *s, const BoxDev &b, const Options &o,
                      cudaStream_t stream)
 {
     k_ccz4_rhs<<<grid_for(b.ivol(), 256), 256, 0, stream>>>(
-        s, b, o, prim, gc, rhs, rcs, inv[0], inv[1], inv[2], st);
+        s, b, o, make_face_opt<double>(o), prim, gc, rhs, rcs, inv[0], inv[1],
+        inv[2], st);
 }
 
 void launch_ccz4_recover(double *s, const BoxDev &b, const Options &o,

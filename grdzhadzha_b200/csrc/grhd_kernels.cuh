@@ -237,6 +237,8 @@ struct EnsMember
     BoxDev sb; // the same box over the RK stage buffer (stride = volume)
     Background bg;
     Options o;
+    FaceOpt<double> fo64; // the face constants of o in the arithmetic type
+    FaceOpt<float> fo32;
     double inv[3];
     double cfl, max_dt;
     double *state, *stage, *acc;
