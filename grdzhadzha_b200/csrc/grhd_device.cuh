@@ -1078,58 +1078,56 @@ GRHD_HD __forceinline__ Cons hlle_flux(const FaceSide &l, const FaceSide &r)
     return f;
 }
 
-// One MUSCL-HLLE face flux between cells L and R (compute_muscl_hlle_flux,
-// FiniteVolume.hpp:63-98, with the face geometry of average_geometry,
-// FArrayBoxFiniteVolume.hpp:194-216).  LL, L, R, RR are the cells
-// i-1, i, i+1, i+2 around face i+1/2.
-GRHD_HD __forceinline__ ConsT<double>
-face_flux(const FaceOpt<double> &o, const PVT<double> &LL,
-          const PVT<double> &L, const PVT<double> &R, const PVT<double> &RR,
-          const GeoT<double> &g, int d)
+GRHD_HD __forceinline__ double slope_of(double l, double c, double r,
+                                        double theta)
 {
-    double ql[5], qr[5];
+    return limited_slope_f64(l, c, r, theta);
+}
+__device__ __forceinline__ float slope_of(float l, float c, float r,
+                                          float theta)
+{
+    return limited_slope(l, c, r, theta);
+}
+
+// The reconstructed values of cell c on its lower and upper faces (MUSCL,
+// Reconstruction.hpp:39-58) from its neighbours l and r along the direction.
+template <typename T>
+GRHD_HD __forceinline__ void cell_states(const FaceOpt<T> &o,
+                                         const PVT<T> &l, const PVT<T> &c,
+                                         const PVT<T> &r, T lower[5],
+                                         T upper[5])
+{
 #pragma unroll
-    for (int c = 0; c < 5; ++c)
+    for (int q = 0; q < 5; ++q)
     {
-        ql[c] = L.q[c];
-        qr[c] = R.q[c];
+        lower[q] = upper[q] = c.q[q];
         if (o.use_recon)
         {
-            ql[c] += 0.5 * limited_slope_f64(LL.q[c], L.q[c], R.q[c], o.theta);
-            qr[c] -= 0.5 * limited_slope_f64(L.q[c], R.q[c], RR.q[c], o.theta);
+            const T s = slope_of(l.q[q], c.q[q], r.q[q], o.theta);
+            upper[q] = c.q[q] + T(0.5) * s;
+            lower[q] = c.q[q] - T(0.5) * s;
         }
     }
+}
+
+// The HLLE flux between the states ql and qr of a face with geometry g.
+GRHD_HD __forceinline__ ConsT<double>
+state_flux(const FaceOpt<double> &o, const double ql[5], const double qr[5],
+           const GeoT<double> &g, int d)
+{
     FaceSide l, r;
     face_side(o, ql, g, d, l);
     face_side(o, qr, g, d, r);
     return hlle_flux(l, r);
 }
 
-// The mixed path's face flux, in the reference's separate formulas.
+// The mixed path's, in the reference's separate formulas.
 __device__ __forceinline__ ConsT<float>
-face_flux(const FaceOpt<float> &o, const PVT<float> &LL, const PVT<float> &L,
-          const PVT<float> &R, const PVT<float> &RR, const GeoT<float> &g,
-          int d)
+state_flux(const FaceOpt<float> &o, const float ql[5], const float qr[5],
+           const GeoT<float> &g, int d)
 {
     using T = float;
     PrimT<T> lp, rp;
-    T ql[5], qr[5];
-#pragma unroll
-    for (int c = 0; c < 5; ++c)
-    {
-        if (o.use_recon)
-        {
-            const T sl = limited_slope(LL.q[c], L.q[c], R.q[c], o.theta);
-            const T sr = limited_slope(L.q[c], R.q[c], RR.q[c], o.theta);
-            ql[c] = L.q[c] + T(0.5) * sl;
-            qr[c] = R.q[c] - T(0.5) * sr;
-        }
-        else
-        {
-            ql[c] = L.q[c];
-            qr[c] = R.q[c];
-        }
-    }
     lp.rho = ql[0];
     lp.p = ql[1];
     rp.rho = qr[0];
@@ -1165,6 +1163,21 @@ face_flux(const FaceOpt<float> &o, const PVT<float> &LL, const PVT<float> &L,
     for (int i = 0; i < 3; ++i)
         f.S[i] = (su * lf.S[i] - sl * rf.S[i] + ss * (rc.S[i] - lc.S[i])) * inv;
     return f;
+}
+
+// One MUSCL-HLLE face flux between cells L and R (compute_muscl_hlle_flux,
+// FiniteVolume.hpp:63-98, with the face geometry of average_geometry,
+// FArrayBoxFiniteVolume.hpp:194-216).  LL, L, R, RR are the cells
+// i-1, i, i+1, i+2 around face i+1/2.
+template <typename T>
+GRHD_HD __forceinline__ ConsT<T>
+face_flux(const FaceOpt<T> &o, const PVT<T> &LL, const PVT<T> &L,
+          const PVT<T> &R, const PVT<T> &RR, const GeoT<T> &g, int d)
+{
+    T ql[5], qr[5], unused[5];
+    cell_states(o, LL, L, R, unused, ql);
+    cell_states(o, L, R, RR, qr, unused);
+    return state_flux(o, ql, qr, g, d);
 }
 
 template <typename T>

@@ -459,52 +459,64 @@ __global__ void __launch_bounds__(256, kMinBlocks<T>)
 
 // ----------------------------------------------------------- face pass
 
+// The tile keeps half of each geometry field a face reads (gamma_ij, the
+// diagonal of gamma^ij, lapse, shift), so the face average of two cells is a
+// sum; halving is exact, so it is the average's value bit for bit.
 template <typename T>
-__device__ __forceinline__ void geo_store(T *g, int n, int cell,
-                                          const GeoT<T> &v)
+__device__ __forceinline__ void geo_store_half(T *g, int n, int cell,
+                                               const GeoT<T> &v)
 {
 #pragma unroll
     for (int s = 0; s < 6; ++s)
-    {
         g[s * n + cell] = v.gLL[s];
-        g[(6 + s) * n + cell] = v.gUU[s];
-    }
-    g[12 * n + cell] = v.lapse;
+    g[6 * n + cell] = v.gUU[0];
+    g[7 * n + cell] = v.gUU[3];
+    g[8 * n + cell] = v.gUU[5];
+    g[9 * n + cell] = v.lapse;
 #pragma unroll
     for (int i = 0; i < 3; ++i)
-        g[(13 + i) * n + cell] = v.shift[i];
+        g[(10 + i) * n + cell] = v.shift[i];
 }
 
 template <typename T>
-__device__ __forceinline__ void geo_load(const T *g, int n, int cell,
-                                         GeoT<T> &v)
+__device__ __forceinline__ void geo_halve(GeoT<T> &v)
 {
 #pragma unroll
     for (int s = 0; s < 6; ++s)
     {
-        v.gLL[s] = g[s * n + cell];
-        v.gUU[s] = g[(6 + s) * n + cell];
+        v.gLL[s] *= T(0.5);
+        v.gUU[s] *= T(0.5);
     }
-    v.lapse = g[12 * n + cell];
+    v.lapse *= T(0.5);
 #pragma unroll
     for (int i = 0; i < 3; ++i)
-        v.shift[i] = g[(13 + i) * n + cell];
+        v.shift[i] *= T(0.5);
 }
 
+// Face geometry along d from two halved cells of the tile.
 template <typename T>
-__device__ __forceinline__ void geo_avg_smem(const T *g, int n, int ca, int cb,
-                                             GeoT<T> &v)
+__device__ __forceinline__ void geo_sum(const T *g, int n, int ca, int cb,
+                                        int d, GeoT<T> &v)
 {
 #pragma unroll
     for (int s = 0; s < 6; ++s)
-    {
-        v.gLL[s] = T(0.5) * (g[s * n + ca] + g[s * n + cb]);
-        v.gUU[s] = T(0.5) * (g[(6 + s) * n + ca] + g[(6 + s) * n + cb]);
-    }
-    v.lapse = T(0.5) * (g[12 * n + ca] + g[12 * n + cb]);
+        v.gLL[s] = g[s * n + ca] + g[s * n + cb];
+    v.gUU[sym(d, d)] = g[(6 + d) * n + ca] + g[(6 + d) * n + cb];
+    v.lapse = g[9 * n + ca] + g[9 * n + cb];
+    v.shift[d] = g[(10 + d) * n + ca] + g[(10 + d) * n + cb];
+}
+
+// The same from a tile cell and a halved cell in registers (z faces).
+template <typename T>
+__device__ __forceinline__ void geo_sum_z(const T *g, int n, int ca,
+                                          const GeoT<T> &b, GeoT<T> &v)
+{
 #pragma unroll
-    for (int i = 0; i < 3; ++i)
-        v.shift[i] = T(0.5) * (g[(13 + i) * n + ca] + g[(13 + i) * n + cb]);
+    for (int s = 0; s < 6; ++s)
+        v.gLL[s] = g[s * n + ca] + b.gLL[s];
+    v.gUU[5] = g[8 * n + ca] + b.gUU[5];
+    v.lapse = g[9 * n + ca] + b.lapse;
+    v.shift[2] = g[12 * n + ca] + b.shift[2];
 }
 
 template <typename T, bool CG = false>
@@ -551,8 +563,7 @@ __device__ __forceinline__ void cp_async_wait_all()
 }
 
 // The primitive cross tile of a z march at plane k (clamped to the
-// ghosted box): synchronous loads, or (ASYNC) cp.async copies completed by
-// cp_async_wait_all before the next barrier.
+// ghosted box): cp.async copies (ASYNC), or loads.
 template <typename T, bool CG, bool ASYNC>
 __device__ __forceinline__ void load_p_tile(T *P, const T *__restrict__ prim,
                                             const BoxDev &b, int i0, int j0,
@@ -575,26 +586,6 @@ __device__ __forceinline__ void load_p_tile(T *P, const T *__restrict__ prim,
             else
                 P[c * nP + idx] = rdro<CG>(&prim[c * b.pcs + g]);
         }
-    }
-}
-
-// Geometry of the cross-shaped (x,y) neighbourhood of a tile at plane kk.
-template <typename T, int BGK = -1>
-__device__ __forceinline__ void tile_geometry(T *G, const Background &bg,
-                                              const Options &o, int i0,
-                                              int j0, int kk, int tid)
-{
-    constexpr int n = kGW * kGW;
-    for (int idx = tid; idx < n; idx += kTB * kTB)
-    {
-        const int u = idx % kGW, v = idx / kGW;
-        if ((u == 0 || u == kGW - 1) && (v == 0 || v == kGW - 1))
-            continue;
-        double x, y, z;
-        cell_xyz(o, i0 - 1 + u, j0 - 1 + v, kk, x, y, z);
-        GeoT<T> g;
-        metric_T<T, false, BGK>(bg, x, y, z, g, nullptr);
-        geo_store(G, n, idx, g);
     }
 }
 
@@ -643,30 +634,49 @@ __device__ __forceinline__ void block_partial(double v, double *scratch,
     }
 }
 
-// 16x16 threads own a 15x15 (x,y) cell tile and march along z over a chunk
-// of planes.  Per plane: the primitive cross tile (2-cell halo) and the
-// geometry cross tile (1-cell halo) in shared memory, geometry double
-// buffered by plane; x and y faces from shared memory (each tile also
-// evaluates its two boundary faces per row), the z face from a 4-plane
-// register window (each z face once); divergence + sources to the RHS.
-// One tile (bx, by, bz) of the face pass; 16x16 threads, `smem_raw` holds
-// faces_smem<T>() bytes; the tile's accretion sum goes to mdot_part[part].
+// 16x16 threads own a 16x16 (x,y) cell tile and march along z over a chunk
+// of planes; every face is evaluated once per tile.  Per plane, two phases
+// between two barriers:
+//   1. the lower x and y face of each thread's cell, from the primitive
+//      tile (2-cell halo, two planes buffered, copied in asynchronously one
+//      plane ahead) and the geometry tile (1-cell halo) in shared memory;
+//      the tile's last x faces fall to warp 0 and its last y faces to warp
+//      1 (the same code once more);
+//   2. the geometry of plane k+1 (own cell in registers and to the tile; the
+//      halo cells fall to warps 2 and 3), the z face above the cell from it,
+//      and the divergence + sources to the RHS.
+// The tile needs one geometry buffer: plane k's x and y faces have read it
+// when plane k+1's cells overwrite it, and a z face reads its own column
+// only.  A cell's z slope serves both its z faces: the upper state is
+// carried to the next plane.  Tiles of 16 cells fit boxes whose sides are
+// multiples of 16 -- the usual patch and grid sizes -- without idle columns.
+// Issue- and latency-bound (FP64 pipe about half busy, DRAM idle): against
+// tiles of 15 cells with three barriers, two geometry buffers and the y
+// fluxes stored across the banks, an FP64 RK4 step of the 256^3 torus went
+// from 24.9 to 21.0 ms (mixed 15.9 to 14.9, results unchanged bit for bit),
+// the 64^3 Michel step from 0.68 to 0.55 ms.
+// The march starts at plane k0-1 (z face only), so the face below k0 comes
+// from the same code as the block below's upper face, bit for bit: the RHS
+// does not depend on where the z blocks start.
+// One tile (bx, by, bz) of the face pass; `smem_raw` holds faces_smem<T>()
+// bytes; the tile's accretion sum goes to mdot_part[part].
 template <typename T, bool MDOT, bool CG = false, int BGK = -1>
 __device__ __forceinline__ void
 faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
            T *__restrict__ rhs, const BoxDev &b, const Background &bg,
-           const Options &o, const FaceOpt<T> &fo, double idx0_, double idx1_, double idx2_,
-           int zchunk, int bx, int by, int bz, unsigned char *smem_raw,
-           double *__restrict__ mdot_part, int64_t part)
+           const Options &o, const FaceOpt<T> &fo, double idx0_, double idx1_,
+           double idx2_, int zchunk, int bx, int by, int bz,
+           unsigned char *smem_raw, double *__restrict__ mdot_part,
+           int64_t part)
 {
-    T *smem = reinterpret_cast<T *>(smem_raw);
     constexpr int nP = kPW * kPW;
     constexpr int nG = kGW * kGW;
-    constexpr int nFx = kTB * kTC; // x faces: a in [0,16), b in [0,15)
-    T *P = smem;                       // [5][nP]
-    T *Gb = P + 5 * nP;                // [2][16][nG]
-    T *Fx = Gb + 2 * kGeoFields * nG;  // [5][nFx]
-    T *Fy = Fx + 5 * nFx;              // [5][nFx]
+    constexpr int nF = kTC * (kTC + 1); // x or y faces of a tile plane
+    constexpr int wX = kTC + 1;         // x faces of a row
+    T *P = reinterpret_cast<T *>(smem_raw); // [2][5][nP]
+    T *G = P + 2 * 5 * nP;                  // [kGeoFields][nG]
+    T *Fx = G + kGeoFields * nG;            // [5][nF], row-major rows of wX
+    T *Fy = Fx + 5 * nF;                    // [5][nF], kTC + 1 rows of kTC
     const T idx0 = T(idx0_), idx1 = T(idx1_), idx2 = T(idx2_);
 
     const int a = threadIdx.x, bb = threadIdx.y;
@@ -676,107 +686,155 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
     const int k0 = b.lo[2] + bz * zchunk;
     const int k1 = min(k0 + zchunk - 1, b.hi[2]);
     const int ci = i0 + a, cj = j0 + bb; // this thread's cell column
-    const bool col_ok = a < kTC && bb < kTC && ci <= b.hi[0] && cj <= b.hi[1];
-    const int ci_c = min(ci, b.hi[0]), cj_c = min(cj, b.hi[1]);
+    const bool col_ok = ci <= b.hi[0] && cj <= b.hi[1];
+    const int64_t plane = (int64_t)b.gn[0] * b.gn[1];
+    const int own_p = (bb + 2) * kPW + a + 2, own_g = (bb + 1) * kGW + a + 1;
+    // this column's primitives at plane k0-2 (clamped into the box)
+    const T *pcol = prim + b.gidx(min(ci, b.hi[0]), min(cj, b.hi[1]), k0 - 2);
 
-    // The z march starts two planes below k0: plane k0-2 only computes
-    // the tile geometry of plane k0-1, plane k0-1 only the z face below
-    // k0.  Every plane's geometry and every z face thus come from the same
-    // code as in the rest of the march, so the face below k0 equals the
-    // block below's upper face bit for bit: the RHS does not depend on
-    // where the z blocks start.  w0..w3 is this column's window
-    // P(k-1 .. k+2) of the z face above plane k.
-    PVT<T> w0, w1, w2, w3;
+    // primitive tiles of planes k0-1 and k0
+    load_p_tile<T, CG, !CG>(P + ((k0 - 1) & 1) * 5 * nP, prim, b, i0, j0,
+                            k0 - 1, tid);
+    load_p_tile<T, CG, !CG>(P + (k0 & 1) * 5 * nP, prim, b, i0, j0, k0, tid);
+    T up[5]; // upper state of the cell at plane k, for the z face above it
+    {
+        T unused[5];
+        cell_states(fo, load_pv_global<T, CG>(pcol, b.pcs, 0),
+                    load_pv_global<T, CG>(pcol, b.pcs, plane),
+                    load_pv_global<T, CG>(pcol, b.pcs, 2 * plane), unused, up);
+    }
+    pcol += 3 * plane; // plane k0+1: plane k+2 of the march's first plane
+
     ConsT<T> Flo = zero_cons<T>();
     double macc = 0.0;
-    w0 = load_pv_global<T, CG>(prim, b.pcs, b.gidx(ci_c, cj_c, k0 - 2));
-    w1 = load_pv_global<T, CG>(prim, b.pcs, b.gidx(ci_c, cj_c, k0 - 1));
-    w2 = load_pv_global<T, CG>(prim, b.pcs, b.gidx(ci_c, cj_c, k0));
-
-    int cur = 0;
+    // k = k0-2 fills the geometry of plane k0-1 only
 #pragma unroll 1
     for (int k = k0 - 2; k <= k1; ++k)
     {
-        T *Gc = Gb + cur * kGeoFields * nG;
-        T *Gn = Gb + (cur ^ 1) * kGeoFields * nG;
+        const T *Pc = P + (k & 1) * 5 * nP;
         const bool zface = k >= k0 - 1; // the z face above plane k
         const bool cells = k >= k0;     // plane k's x/y faces and RHS
+        if (cells)
+        {
+            // x face between cells (i0+fa-1, i0+fa) in row j0+fb
+#pragma unroll 1
+            for (int pass = 0; pass < 2; ++pass)
+            {
+                const int fa = pass ? kTC : a, fb = pass ? tid : bb;
+                if (pass && tid >= kTC)
+                    break;
+                if (j0 + fb > b.hi[1] || i0 + fa - 1 > b.hi[0])
+                    continue;
+                const int row = (fb + 2) * kPW + fa;
+                GeoT<T> gf;
+                geo_sum(G, nG, (fb + 1) * kGW + fa, (fb + 1) * kGW + fa + 1, 0,
+                        gf);
+                const ConsT<T> f = face_flux(
+                    fo, load_pv_smem(Pc, row), load_pv_smem(Pc, row + 1),
+                    load_pv_smem(Pc, row + 2), load_pv_smem(Pc, row + 3), gf,
+                    0);
+                const int fi = fb * wX + fa;
+                if (MDOT && fa < kTC && i0 + fa <= b.hi[0])
+                    macc +=
+                        mdot_face(o, i0 + fa - 1, j0 + fb, k, 0, gf, f.D);
+                Fx[0 * nF + fi] = f.D;
+                Fx[1 * nF + fi] = f.S[0];
+                Fx[2 * nF + fi] = f.S[1];
+                Fx[3 * nF + fi] = f.S[2];
+                Fx[4 * nF + fi] = f.tau;
+            }
+            // y face between rows (j0+fb-1, j0+fb) in column i0+fa
+#pragma unroll 1
+            for (int pass = 0; pass < 2; ++pass)
+            {
+                const int fa = pass ? tid - 32 : a, fb = pass ? kTC : bb;
+                if (pass && (unsigned)fa >= (unsigned)kTC)
+                    break;
+                if (i0 + fa > b.hi[0] || j0 + fb - 1 > b.hi[1])
+                    continue;
+                const int col = fb * kPW + fa + 2;
+                GeoT<T> gf;
+                geo_sum(G, nG, fb * kGW + fa + 1, (fb + 1) * kGW + fa + 1, 1,
+                        gf);
+                const ConsT<T> f = face_flux(
+                    fo, load_pv_smem(Pc, col), load_pv_smem(Pc, col + kPW),
+                    load_pv_smem(Pc, col + 2 * kPW),
+                    load_pv_smem(Pc, col + 3 * kPW), gf, 1);
+                const int fi = fb * kTC + fa;
+                if (MDOT && fb < kTC && j0 + fb <= b.hi[1])
+                    macc +=
+                        mdot_face(o, i0 + fa, j0 + fb - 1, k, 1, gf, f.D);
+                Fy[0 * nF + fi] = f.D;
+                Fy[1 * nF + fi] = f.S[0];
+                Fy[2 * nF + fi] = f.S[1];
+                Fy[3 * nF + fi] = f.S[2];
+                Fy[4 * nF + fi] = f.tau;
+            }
+        }
+        // this column's primitives at planes k and k+2 of the face above
+        PVT<T> w1, w3;
         if (zface)
-            w3 = load_pv_global<T, CG>(prim, b.pcs, b.gidx(ci_c, cj_c, k + 2));
-        // primitive cross tile at plane k: issued after the previous
-        // plane's faces (asynchronous copies, overlapping that plane's
-        // output and this plane's geometry), or loaded here (the ensemble's
-        // coherent loads)
-        if (cells && CG)
-            load_p_tile<T, CG, false>(P, prim, b, i0, j0, k, tid);
-        tile_geometry<T, BGK>(Gn, bg, o, i0, j0, k + 1, tid);
-        if (cells && !CG)
+        {
+            w1 = load_pv_smem(Pc, own_p);
+            w3 = load_pv_global<T, CG>(pcol, b.pcs, 0);
+            pcol += plane;
+        }
+        // plane k+1's tile, issued one plane ago (the first two before the
+        // march), has landed
+        if (!CG)
             cp_async_wait_all();
         __syncthreads();
-
-        // x face between cells (i0+a-1, i0+a) in row j0+bb
-        if (cells && bb < kTC && cj <= b.hi[1] && i0 + a - 1 <= b.hi[0])
+        // plane k's tile has been read: fetch plane k+2's into its place
+        // (of plane k1+1 the z faces read their own columns)
+        if (zface && k < k1)
+            load_p_tile<T, CG, !CG>(P + (k & 1) * 5 * nP, prim, b, i0, j0,
+                                    k + 2, tid);
+        // geometry of plane k+1: the halo cells (where the next plane has x
+        // and y faces), then the own cell, left in registers
+        GeoT<T> gn;
+        const int halo = tid - 64;
+        const bool has_halo =
+            (unsigned)halo < 4u * kTC && zface && k + 1 <= k1;
+#pragma unroll 1
+        for (int pass = has_halo ? 0 : 1; pass < 2; ++pass)
         {
-            const int row = (bb + 2) * kPW;
-            GeoT<T> gf;
-            geo_avg_smem(Gc, nG, (bb + 1) * kGW + a, (bb + 1) * kGW + a + 1, gf);
-            const ConsT<T> f = face_flux(fo, load_pv_smem(P, row + a),
-                                         load_pv_smem(P, row + a + 1),
-                                         load_pv_smem(P, row + a + 2),
-                                         load_pv_smem(P, row + a + 3), gf, 0);
-            const int fi = bb * kTB + a;
-            if (MDOT && a < kTC && i0 + a <= b.hi[0])
-                macc += mdot_face(o, i0 + a - 1, cj, k, 0, gf, f.D);
-            Fx[0 * nFx + fi] = f.D;
-            Fx[1 * nFx + fi] = f.S[0];
-            Fx[2 * nFx + fi] = f.S[1];
-            Fx[3 * nFx + fi] = f.S[2];
-            Fx[4 * nFx + fi] = f.tau;
-        }
-        // y face between rows (j0+bb-1, j0+bb) in column i0+a
-        if (cells && a < kTC && ci <= b.hi[0] && j0 + bb - 1 <= b.hi[1])
-        {
-            GeoT<T> gf;
-            geo_avg_smem(Gc, nG, bb * kGW + a + 1, (bb + 1) * kGW + a + 1, gf);
-            const int col = a + 2;
-            const ConsT<T> f = face_flux(fo, load_pv_smem(P, bb * kPW + col),
-                                         load_pv_smem(P, (bb + 1) * kPW + col),
-                                         load_pv_smem(P, (bb + 2) * kPW + col),
-                                         load_pv_smem(P, (bb + 3) * kPW + col),
-                                         gf, 1);
-            const int fi = a * kTB + bb;
-            if (MDOT && bb < kTC && j0 + bb <= b.hi[1])
-                macc += mdot_face(o, ci, j0 + bb - 1, k, 1, gf, f.D);
-            Fy[0 * nFx + fi] = f.D;
-            Fy[1 * nFx + fi] = f.S[0];
-            Fy[2 * nFx + fi] = f.S[1];
-            Fy[3 * nFx + fi] = f.S[2];
-            Fy[4 * nFx + fi] = f.tau;
+            int u = a + 1, v = bb + 1;
+            if (pass == 0)
+            {
+                const int at = halo % kTC + 1;
+                u = halo < 2 * kTC ? (halo < kTC ? 0 : kGW - 1) : at;
+                v = halo < 2 * kTC ? at : (halo < 3 * kTC ? 0 : kGW - 1);
+            }
+            double x, y, z;
+            cell_xyz(o, i0 - 1 + u, j0 - 1 + v, k + 1, x, y, z);
+            metric_T<T, false, BGK>(bg, x, y, z, gn, nullptr);
+            geo_halve(gn);
+            if (pass == 0)
+                geo_store_half(G, nG, v * kGW + u, gn);
         }
         // z face at k+1/2 for this column
         ConsT<T> Fhi = zero_cons<T>();
         if (zface && col_ok)
         {
-            GeoT<T> gf, gA, gB;
-            const int cell = (bb + 1) * kGW + a + 1;
-            geo_load(Gc, nG, cell, gA);
-            geo_load(Gn, nG, cell, gB);
-            average_geo(gA, gB, gf);
-            Fhi = face_flux(fo, w0, w1, w2, w3, gf, 2);
+            GeoT<T> gf;
+            geo_sum_z(G, nG, own_g, gn, gf);
+            const PVT<T> w2 = load_pv_smem(P + ((k + 1) & 1) * 5 * nP, own_p);
+            T low[5], next[5];
+            cell_states(fo, w1, w2, w3, low, next);
+            Fhi = state_flux(fo, up, low, gf, 2);
+#pragma unroll
+            for (int c = 0; c < 5; ++c)
+                up[c] = next[c];
             // a box counts the sphere faces whose upper cell it holds, in
             // every direction, so the boxes of a level count each once
             if (MDOT && (cells ? k < b.hi[2] : k0 == b.lo[2]))
                 macc += mdot_face(o, ci, cj, k, 2, gf, Fhi.D);
         }
-        __syncthreads();
-        // the x/y faces have read plane k's tile: fetch plane k+1's
-        if (!CG && k + 1 >= k0 && k + 1 <= k1)
-            load_p_tile<T, CG, true>(P, prim, b, i0, j0, k + 1, tid);
+        geo_store_half(G, nG, own_g, gn);
 
         if (cells && col_ok)
         {
-            const int fxl = bb * kTB + a, fxh = bb * kTB + a + 1;
-            const int fyl = a * kTB + bb, fyh = a * kTB + bb + 1;
+            const int fx = bb * wX + a, fy = bb * kTC + a;
             const int64_t ri = b.iidx(ci, cj, k);
             T out[5];
             const T fl[5] = {Flo.D, Flo.S[0], Flo.S[1], Flo.S[2], Flo.tau};
@@ -784,8 +842,9 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
 #pragma unroll
             for (int c = 0; c < 5; ++c)
             {
-                const T rx = -idx0 * (Fx[c * nFx + fxh] - Fx[c * nFx + fxl]);
-                const T ry = -idx1 * (Fy[c * nFx + fyh] - Fy[c * nFx + fyl]);
+                const T rx = -idx0 * (Fx[c * nF + fx + 1] - Fx[c * nF + fx]);
+                const T ry =
+                    -idx1 * (Fy[c * nF + fy + kTC] - Fy[c * nF + fy]);
                 const T rz = -idx2 * (fh[c] - fl[c]);
                 out[c] = ((rx + ry) + rz) + rdro<CG>(&src[c * b.rcs + ri]);
             }
@@ -800,13 +859,6 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
                 rhs[c * b.rcs + ri] = out[c];
         }
         Flo = Fhi;
-        if (zface)
-        {
-            w0 = w1;
-            w1 = w2;
-            w2 = w3;
-        }
-        cur ^= 1;
         __syncthreads();
     }
     if (MDOT)
@@ -1771,7 +1823,8 @@ int grid_for(int64_t n, int threads)
 template <typename T> size_t faces_smem()
 {
     return sizeof(T) *
-           (5 * kPW * kPW + 2 * kGeoFields * kGW * kGW + 2 * 5 * kTB * kTC);
+           (2 * 5 * kPW * kPW + kGeoFields * kGW * kGW +
+            2 * 5 * kTC * (kTC + 1));
 }
 
 // ---------------------------------------------- CCZ4-stored geometry
@@ -2305,17 +2358,42 @@ int64_t face_makespan(int64_t nf, int64_t df, int64_t np, int64_t dp,
     return end;
 }
 
+// The march length of a launch: of the candidates, the one whose blocks,
+// list-scheduled in launch order on the resident slots, finish first (ties
+// keep the longer march).  A block costs its planes and, once, the two
+// lead-in planes (one z face and two planes' geometry): 0.7 of a plane.
+// Marches down to one plane spread a small box over the idle SMs: a plane
+// takes one block about 9 us, whatever the box (a 16^3 right-hand side:
+// 102 us with at least four planes a block, 58 with one; 45x38x31: 84, 70).
 int face_zchunk(const BoxDev &b, int zchunk, bool fp32)
 {
     if (zchunk > 0)
         return zchunk;
-    return face_zchunk_model(b.in[0], b.in[1], b.in[2], face_slots(fp32));
+    const int64_t slots = face_slots(fp32);
+    const int64_t tiles = (int64_t)((b.in[0] + kTC - 1) / kTC) *
+                          ((b.in[1] + kTC - 1) / kTC);
+    const int cand[] = {48, 40, 32, 24, 20, 16, 13, 12, 11, 10,
+                        9,  8,  7,  6,  5,  4,  3,  2,  1};
+    int best = 1;
+    int64_t best_cost = -1;
+    for (int z : cand)
+    {
+        const int r = b.in[2] % z;
+        const int64_t cost =
+            face_makespan(tiles * (b.in[2] / z), 10 * z + 7, r ? tiles : 0,
+                          10 * r + 7, slots);
+        if (best_cost < 0 || cost < best_cost)
+        {
+            best = z;
+            best_cost = cost;
+        }
+    }
+    return best;
 }
 
 int face_zchunk_model(int nx, int ny, int nz, int64_t slots)
 {
-    const int64_t tiles =
-        (int64_t)((nx + kTC - 1) / kTC) * ((ny + kTC - 1) / kTC);
+    const int64_t tiles = (int64_t)((nx + 14) / 15) * ((ny + 14) / 15);
     const int cand[5] = {32, 16, 8, 6, 4};
     int best = cand[0];
     int64_t best_cost = -1;

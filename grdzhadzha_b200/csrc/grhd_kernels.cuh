@@ -127,26 +127,26 @@ enum : int
     kV1 = 8
 };
 
-// Face kernel tiling: 16x16 threads own a 15x15 cell tile in (x, y) and
+// Face kernel tiling: 16x16 threads own a 16x16 cell tile in (x, y) and
 // march along z.
 constexpr int kTB = 16;
-constexpr int kTC = 15;
+constexpr int kTC = 16;
 constexpr int kPW = kTC + 4; // primitive tile width (2 halo each side)
 constexpr int kGW = kTC + 2; // geometry tile width (1 halo each side)
-constexpr int kGeoFields = 16;
+constexpr int kGeoFields = 13; // gamma_ij, diag gamma^ij, lapse, shift
 
 // Per-device kernel attributes (dynamic shared memory of the face kernels).
 cudaError_t configure_kernels();
 // z-march length (planes per block) of the face kernel for box b: zchunk
-// when positive; otherwise face_zchunk_model with the device's resident
-// face blocks (SMs x the occupancy query's blocks per SM).
+// when positive, else the length whose launch finishes first (the RHS does
+// not depend on it).
 int face_zchunk(const BoxDev &b, int zchunk, bool fp32);
-// Of 32, 16, 8, 6 and 4 planes, the one whose launch has the shortest
-// makespan when its blocks -- every full z block of every (x,y) tile, then
-// the short last z row -- are list-scheduled in launch order on `slots`
-// resident blocks, a block costing its planes plus its two lead-in planes
-// (ties keep the longer march).  Host only; the RHS does not depend on the
-// choice.
+// The C entry point's schedule estimate, for tiles of 15 cells and of 32,
+// 16, 8, 6 and 4 planes: the length with the shortest makespan when the
+// launch's blocks -- every full z block of every (x,y) tile, then the short
+// last z row -- are list-scheduled in launch order on `slots` resident
+// blocks, a block costing its planes plus two lead-in planes (ties keep the
+// longer march).  Host only.
 int face_zchunk_model(int nx, int ny, int nz, int64_t slots);
 int64_t face_kernel_blocks(const BoxDev &b, int zchunk, bool fp32 = false);
 
