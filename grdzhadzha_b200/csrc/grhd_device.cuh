@@ -125,7 +125,18 @@ GRHD_HD __forceinline__ double sqrt_(double a)
 #endif
 }
 __device__ __forceinline__ float sqrt_(float a) { return sqrtf(a); }
-// 1/a and 1/sqrt(a) within about one ulp, for the face fluxes: one step of
+// A product that is never fused into a following sum.  Code shared by
+// kernels that must agree bit for bit writes its sums as fma() and its
+// products as mul_(), so that no compiler choice of fused pairs is left.
+GRHD_HD __forceinline__ double mul_(double a, double b)
+{
+#ifdef __CUDA_ARCH__
+    return __dmul_rn(a, b);
+#else
+    return a * b;
+#endif
+}
+// 1/a and 1/sqrt(a) within about one ulp: one step of
 // the third-order iteration (Householder's) from the approximate value y0 of
 // relative error d <= 2^-20: with e = 1 - a y0, 1/a = y0 (1 + e + e^2) up to
 // d^3; with e = 1 - a y0^2, a^-1/2 = y0 (1 + e/2 + 3 e^2/8) up to d^3.  Three
@@ -688,13 +699,13 @@ GRHD_HD __forceinline__ double c2p_S2(const Cons &c, const double gUU[6])
 }
 
 // The primitives of a converged pressure, Valencia.hpp:213-226; false when
-// the velocity reaches the cap.
+// the velocity reaches the cap.  mU = gamma^ij S_j, S2 = S_i mU^i.
 GRHD_HD __forceinline__ bool c2p_finish(const Options &o, const Cons &c,
-                                           const double gUU[6], double S2,
-                                           double p, Prim &out)
+                                        const double mU[3], double S2,
+                                        double p, Prim &out)
 {
     const double e = c.tau + c.D + p;
-    const double v2 = div_(S2, e * e);
+    const double v2 = div_(S2, mul_(e, e));
     if (!(v2 < o.rec_vmax2))
         return false;
     // W rounded as the reference's 1 / sqrt(1 - v^2) (sqrt_ and rcp_ give
@@ -704,16 +715,163 @@ GRHD_HD __forceinline__ bool c2p_finish(const Options &o, const Cons &c,
     const double W = rcp_(sqrt_(1.0 - v2));
     out.rho = div_(c.D, W);
     out.p = p;
-    out.eps = div_(p, (o.G - 1.0) * out.rho);
+    out.eps = div_(p, mul_(o.G - 1.0, out.rho));
     const double ie = rcp_(e);
-    out.v[0] = (gUU[0] * c.S[0] + gUU[1] * c.S[1] + gUU[2] * c.S[2]) * ie;
-    out.v[1] = (gUU[1] * c.S[0] + gUU[3] * c.S[1] + gUU[4] * c.S[2]) * ie;
-    out.v[2] = (gUU[2] * c.S[0] + gUU[4] * c.S[1] + gUU[5] * c.S[2]) * ie;
+    out.v[0] = mul_(mU[0], ie);
+    out.v[1] = mul_(mU[1], ie);
+    out.v[2] = mul_(mU[2], ie);
     return true;
 }
 
-// recover_primitive, Valencia.hpp:116-228 (bounded loops throughout).
+// gamma^ij S_j
+GRHD_HD __forceinline__ void raise(const double gUU[6], const double S[3],
+                                   double mU[3])
+{
+    mU[0] = fma(gUU[0], S[0], fma(gUU[1], S[1], mul_(gUU[2], S[2])));
+    mU[1] = fma(gUU[1], S[0], fma(gUU[3], S[1], mul_(gUU[4], S[2])));
+    mU[2] = fma(gUU[2], S[0], fma(gUU[4], S[1], mul_(gUU[5], S[2])));
+}
+
+GRHD_HD __forceinline__ double dot3(const double a[3], const double b[3])
+{
+    return fma(a[0], b[0], fma(a[1], b[1], mul_(a[2], b[2])));
+}
+
+// The residual of c2p_residual and its derivative with one-ulp reciprocals;
+// tD = tau + D.
+GRHD_HD __forceinline__ double c2p_f(double p, double D, double tD, double S2,
+                                     double Gfac, double vmax2, double &deriv)
+{
+    const double e = tD + p;
+    const double ie = rcp_ulp(e);
+    double v2 = mul_(mul_(S2, ie), ie);
+    if (v2 > vmax2)
+        v2 = vmax2;
+    const double W = rsqrt_ulp(1.0 - v2);
+    const double W2 = mul_(W, W), DW = mul_(D, W), GW2 = mul_(Gfac, W2);
+    // dW/dp = -W t with t = W^2 v^2 / e
+    const double t = mul_(mul_(W2, v2), ie);
+    deriv = fma(-DW, t, fma(GW2, fma(-2.0 * p, t, 1.0), -1.0));
+    return fma(GW2, p, DW) - e;
+}
+
+// The root solve of recover_primitive, Valencia.hpp:116-228 (bounded loops
+// throughout): the reference's bracket, start and accepted iterate.  Its
+// chain of dependent FP64 operations is what it costs, so the residuals at
+// the pressure floor and at the start, which do not depend on one another,
+// are evaluated side by side, and the residual at the bracket's upper end
+// only where its sign is not known: with u >= |tau| and W >= 1,
+// f(u) >= (G/(G-1) - 1) u - tau >= u/4 for G/(G-1) >= 9/4 (G <= 9/5), far
+// above rounding.
+GRHD_HD __forceinline__ bool c2p_solve(const Options &o, const Cons &c,
+                                       double S2, double &p_out, int &iters,
+                                       double &resid)
+{
+    iters = 0;
+    resid = 0.0;
+    if (!(c.D > 0.0))
+        return false;
+    const double Gm1 = o.G - 1.0;
+    const double Gfac = div_(o.G, Gm1);
+    const double vmax2 = o.rec_vmax2;
+    const double tol = o.rec_tol;
+    const double tD = c.tau + c.D;
+    double lower = o.rec_pfloor;
+    double upper = fmax(1.0, fabs(c.tau) + c.D);
+    double dres, dlow;
+    const double f_lower = c2p_f(lower, c.D, tD, S2, Gfac, vmax2, dlow);
+    double p = fmin(fmax(mul_(c.tau, Gm1), lower), upper);
+    double r = c2p_f(p, c.D, tD, S2, Gfac, vmax2, dres);
+    const bool at_floor = fabs(f_lower) <= tol;
+    if (!(f_lower < 0.0) && !at_floor)
+    {
+        // no root above the floor (or not a number)
+        resid = f_lower >= 0.0 ? 0.0 : f_lower;
+        return false;
+    }
+    const bool bracketed = f_lower < 0.0;
+    if (!bracketed)
+        upper = lower;
+    else if (!(Gfac >= 2.25) || !isfinite(upper))
+    {
+        double du;
+        double f_upper = c2p_f(upper, c.D, tD, S2, Gfac, vmax2, du);
+        for (int b = 0; f_upper <= 0.0 && b < o.rec_maxit; ++b)
+        {
+            upper *= 2.0;
+            f_upper = c2p_f(upper, c.D, tD, S2, Gfac, vmax2, du);
+        }
+        if (!(f_upper > 0.0))
+            return false;
+        // the start is clamped to the widened bracket
+        if (!at_floor)
+        {
+            p = fmin(fmax(mul_(c.tau, Gm1), lower), upper);
+            r = c2p_f(p, c.D, tD, S2, Gfac, vmax2, dres);
+        }
+    }
+    if (at_floor)
+    {
+        p = lower;
+        r = f_lower;
+        dres = dlow;
+    }
+    for (int it = 0; it < o.rec_maxit; ++it)
+    {
+        iters = it + 1;
+        if (fabs(r) < tol)
+            break;
+        if (bracketed)
+        {
+            if (r > 0.0)
+                upper = p;
+            else
+                lower = p;
+        }
+        double np = fma(-r, rcp_ulp(dres), p);
+        if (!isfinite(np) || np <= lower || np >= upper)
+            np = 0.5 * (lower + upper);
+        p = np;
+        r = c2p_f(p, c.D, tD, S2, Gfac, vmax2, dres);
+    }
+    resid = r;
+    p_out = p;
+    return fabs(r) < tol;
+}
+
+// recover_primitive, Valencia.hpp:116-228.
 GRHD_HD __forceinline__ bool con2prim(const Options &o, const Cons &c,
+                                         const double gUU[6], Prim &out,
+                                         int *iters_out, double *resid_out)
+{
+    double mU[3], p = 0.0, resid;
+    int iters;
+    raise(gUU, c.S, mU);
+    const double S2 = dot3(c.S, mU);
+    const bool ok = c2p_solve(o, c, S2, p, iters, resid) &&
+                    c2p_finish(o, c, mU, S2, p, out);
+    if (iters_out)
+        *iters_out = iters;
+    if (resid_out)
+        *resid_out = resid;
+    return ok;
+}
+
+GRHD_HD __forceinline__ bool c2p_finish_gUU(const Options &o, const Cons &c,
+                                            const double gUU[6], double S2,
+                                            double p, Prim &out)
+{
+    const double mU[3] = {
+        gUU[0] * c.S[0] + gUU[1] * c.S[1] + gUU[2] * c.S[2],
+        gUU[1] * c.S[0] + gUU[3] * c.S[1] + gUU[4] * c.S[2],
+        gUU[2] * c.S[0] + gUU[4] * c.S[1] + gUU[5] * c.S[2]};
+    return c2p_finish(o, c, mU, S2, p, out);
+}
+
+// The mixed path's bracketed solve: the same root solve one residual at a
+// time.  Its kernels hold three blocks per SM at 80 registers, where
+// c2p_solve's overlapped residuals spill (stage kernel: 224 -> 356 bytes).
+GRHD_HD __forceinline__ bool con2prim_mixed(const Options &o, const Cons &c,
                                          const double gUU[6], Prim &out,
                                          int *iters_out, double *resid_out)
 {
@@ -772,7 +930,7 @@ GRHD_HD __forceinline__ bool con2prim(const Options &o, const Cons &c,
             }
             resid = r;
             if (fabs(r) < tol)
-                ok = c2p_finish(o, c, gUU, S2, p, out);
+                ok = c2p_finish_gUU(o, c, gUU, S2, p, out);
         }
     }
     if (iters_out)
@@ -801,8 +959,8 @@ GRHD_HD __forceinline__ bool con2prim_warm(const Options &o, const Cons &c,
         const double r = c2p_residual(o.rec_pfloor, c.D, c.tau, S2, G,
                                       div_(G, G - 1.0), o.rec_vmax2, nullptr);
         if (fabs(r) <= o.rec_tol)
-            return c2p_finish(o, c, gUU, S2, o.rec_pfloor, out) ||
-                   con2prim(o, c, gUU, out, nullptr, nullptr);
+            return c2p_finish_gUU(o, c, gUU, S2, o.rec_pfloor, out) ||
+                   con2prim_mixed(o, c, gUU, out, nullptr, nullptr);
     }
     if (c.D > 0.0 && p_guess > o.rec_pfloor && isfinite(p_guess))
     {
@@ -814,8 +972,8 @@ GRHD_HD __forceinline__ bool con2prim_warm(const Options &o, const Cons &c,
         for (int it = 0; it < 6; ++it)
         {
             if (fabs(r) < o.rec_tol)
-                return c2p_finish(o, c, gUU, S2, p, out) ||
-                       con2prim(o, c, gUU, out, nullptr, nullptr);
+                return c2p_finish_gUU(o, c, gUU, S2, p, out) ||
+                       con2prim_mixed(o, c, gUU, out, nullptr, nullptr);
             const double np = p - div_(r, dres);
             if (!isfinite(np) || !(np > o.rec_pfloor))
                 break;
@@ -823,7 +981,7 @@ GRHD_HD __forceinline__ bool con2prim_warm(const Options &o, const Cons &c,
             r = c2p_residual(p, c.D, c.tau, S2, G, Gfac, o.rec_vmax2, &dres);
         }
     }
-    return con2prim(o, c, gUU, out, nullptr, nullptr);
+    return con2prim_mixed(o, c, gUU, out, nullptr, nullptr);
 }
 
 // enforce_primitive_floors, Atmosphere.hpp:24-46 (eps recomputed always);
@@ -1268,6 +1426,229 @@ GRHD_HD __forceinline__ ConsT<T> static_sources(const PrimT<T> &pr,
         s.S[m] = ms;
     }
     return s;
+}
+
+// -------------------------------------------- FP64 Kerr-Schild cell
+// The per-cell work of the FP64 path on a Kerr-Schild hole in terms of the
+// null vector l and H: gamma_ij = delta_ij + F l_i l_j (F = 2H),
+// gamma^ij = delta^ij - c l_i l_j, beta^i = c l^i, with alpha^2 = 1/(1 + F)
+// and c = F alpha^2 (l.l = 1).  Ten numbers instead of the 55 of GeoFullT
+// are live across the recovery, and the sources contract the derivatives of
+// H and l with the fluid directly (ks_sources).  Sums are fma() and products
+// mul_(): every kernel that calls these gets the same bits.
+// The stage kernel was bound by the spills of those 55 values (580 MB of
+// local stores at 128^3) and by the length of the recovery's chain; with
+// this, c2p_solve and 32-bit cell indices it holds 128 registers without a
+// spill: 2.77 -> 1.55 ms per launch at 256^3 (bytes alone: 0.72), the RK4
+// step 21.0 -> 15.8 ms.
+struct KsCell
+{
+    double l[3], F, c, alpha, alpha2;
+    double r, inv_r, inv_ra, inv_sigma; // 1/r, 1/(r^2 + a^2), 1/Sigma
+};
+
+GRHD_HD __forceinline__ void ks_cell(double M, double a, double x, double y,
+                                     double z, KsCell &k)
+{
+    const double a2 = mul_(a, a);
+    const double rho2 =
+        fmax(fma(x, x, fma(y, y, mul_(z, z))), 1.0e-12); // (1e-6)^2
+    const double hA = 0.5 * (rho2 - a2);
+    const double az = mul_(a, z);
+    const double r2 = hA + sqrt_(fma(hA, hA, mul_(az, az)));
+    // r and 1/r from one reciprocal square root, each corrected once
+    const double y0 = rsqrt_ulp(r2);
+    const double r0 = mul_(r2, y0);
+    const double r = fma(fma(-r0, r0, r2), 0.5 * y0, r0);
+    k.r = r;
+    k.inv_r = fma(fma(-r, y0, 1.0), y0, y0);
+    const double ct = mul_(z, k.inv_r);
+    const double act = mul_(a, ct);
+    k.inv_sigma = rcp_ulp(fma(act, act, r2));
+    k.inv_ra = rcp_ulp(r2 + a2);
+    k.l[0] = mul_(fma(r, x, mul_(a, y)), k.inv_ra);
+    k.l[1] = mul_(fma(r, y, -mul_(a, x)), k.inv_ra);
+    k.l[2] = ct;
+    k.F = mul_(mul_(2.0 * M, r), k.inv_sigma);
+    const double u = 1.0 + k.F;
+    k.alpha2 = rcp_ulp(u);
+    k.alpha = rsqrt_ulp(u);
+    k.c = mul_(k.F, k.alpha2);
+}
+
+// gamma^ij S_j
+GRHD_HD __forceinline__ void ks_raise(const KsCell &k, const double S[3],
+                                      double mU[3])
+{
+    const double t = mul_(k.c, dot3(k.l, S));
+    mU[0] = fma(-t, k.l[0], S[0]);
+    mU[1] = fma(-t, k.l[1], S[1]);
+    mU[2] = fma(-t, k.l[2], S[2]);
+}
+
+GRHD_HD __forceinline__ double ks_vsq(const KsCell &k, const double v[3])
+{
+    const double lv = dot3(k.l, v);
+    return fma(mul_(k.F, lv), lv, dot3(v, v));
+}
+
+// enforce_primitive_floors (floors), Atmosphere.hpp:24-46
+GRHD_HD __forceinline__ void ks_floors(const Options &o, const KsCell &k,
+                                       Prim &pr)
+{
+    pr.rho = fmax(pr.rho, o.rho_floor);
+    pr.p = fmax(pr.p, o.p_floor);
+    const double v2 = ks_vsq(k, pr.v);
+    if (v2 >= o.atmo_vmax2)
+    {
+        const double s = sqrt_(div_(o.atmo_vmax2, v2));
+        pr.v[0] = mul_(pr.v[0], s);
+        pr.v[1] = mul_(pr.v[1], s);
+        pr.v[2] = mul_(pr.v[2], s);
+    }
+    pr.eps = div_(pr.p, mul_(o.G - 1.0, pr.rho));
+}
+
+GRHD_HD __forceinline__ void ks_gLL(const KsCell &k, double g[6])
+{
+    const double f[3] = {mul_(k.F, k.l[0]), mul_(k.F, k.l[1]),
+                         mul_(k.F, k.l[2])};
+    g[0] = fma(f[0], k.l[0], 1.0);
+    g[1] = mul_(f[0], k.l[1]);
+    g[2] = mul_(f[0], k.l[2]);
+    g[3] = fma(f[1], k.l[1], 1.0);
+    g[4] = mul_(f[1], k.l[2]);
+    g[5] = fma(f[2], k.l[2], 1.0);
+}
+
+GRHD_HD __forceinline__ bool ks_con2prim(const Options &o, const KsCell &k,
+                                         const Cons &c, Prim &out)
+{
+    double mU[3], p, resid;
+    int iters;
+    ks_raise(k, c.S, mU);
+    const double S2 = dot3(c.S, mU);
+    return c2p_solve(o, c, S2, p, iters, resid) &&
+           c2p_finish(o, c, mU, S2, p, out);
+}
+
+// compute_static_metric_source_terms (static_sources, StaticMetric.hpp:
+// 193-275) at a Kerr-Schild cell, contracted by hand.  With D_i = d_i H:
+//   d_i alpha = -alpha^3 D_i, d_i beta^j = 2 alpha^4 D_i l^j + c d_i l^j,
+//   d_i ln sqrt(gamma) = alpha^2 D_i,
+//   d_m gamma_ij = 2 D_m l_i l_j + F (l_i d_m l_j + l_j d_m l_i),
+//   l.d_m l = 0, l^m d_m l_i = 0 (l is unit and geodesic),
+// and d_i r = (r x_i + a^2 z delta_iz / r) / Sigma, so that for any vector u
+//   u.d_i l = d_i r w(u) + ((r u_x - a u_y) delta_ix + (r u_y + a u_x)
+//             delta_iy) / (r^2 + a^2) + u_z delta_iz / r,
+//   w(u) = (u_x (x - 2 r l_x) + u_y (y - 2 r l_y)) / (r^2 + a^2)
+//          - u_z l_z / r.
+GRHD_HD __forceinline__ Cons ks_sources(const Options &o, double a,
+                                        const KsCell &k, double x, double y,
+                                        double z, const Prim &pr,
+                                        const Cons &c)
+{
+    const double a2 = mul_(a, a);
+    const double *l = k.l, *v = pr.v;
+    // d r, d H
+    const double rs = mul_(k.r, k.inv_sigma);
+    const double ias = mul_(k.inv_r, k.inv_sigma);
+    const double dr[3] = {mul_(rs, x), mul_(rs, y),
+                          mul_(fma(a2, ias, rs), z)};
+    const double H = 0.5 * k.F;
+    const double a2ct = mul_(a2, l[2]);
+    // r - a^2 ct^2 / r
+    const double rm = fma(-mul_(a2ct, l[2]), k.inv_r, k.r);
+    const double hk = mul_(H, fma(mul_(-2.0, k.inv_sigma), rm, k.inv_r));
+    const double dH[3] = {mul_(hk, dr[0]), mul_(hk, dr[1]),
+                          fma(hk, dr[2], -mul_(mul_(k.F, a2ct), ias))};
+    const double vH = dot3(v, dH), lH = dot3(l, dH);
+    double mU[3];
+    ks_raise(k, c.S, mU);
+    const double mH = dot3(mU, dH), Sl = dot3(c.S, l);
+    // rho h W^2, v.l
+    const double lv = dot3(l, v);
+    const double vv = fma(mul_(k.F, lv), lv, dot3(v, v));
+    const double rhw = mul_(mul_(pr.rho, fma(o.G, pr.eps, 1.0)),
+                            rcp_ulp(1.0 - vv));
+    const double rl = mul_(rhw, lv);
+    // l_i T^ij l_j of the stress T^ij = rhw v^i v^j + p gamma^ij
+    const double lTl = fma(rl, lv, mul_(pr.p, k.alpha2));
+    // transport velocity along d ln sqrt(gamma)
+    const double T =
+        mul_(k.alpha2, fma(k.alpha, vH, -mul_(k.c, lH)));
+    // w(u), v.dl.v and div l
+    const double tr = 2.0 * k.r;
+    const double wx = mul_(fma(-tr, l[0], x), k.inv_ra);
+    const double wy = mul_(fma(-tr, l[1], y), k.inv_ra);
+    const double wz = -mul_(l[2], k.inv_r);
+    const double ri = mul_(k.r, k.inv_ra);
+    const double wv = fma(v[0], wx, fma(v[1], wy, mul_(v[2], wz)));
+    const double vA =
+        fma(dot3(v, dr), wv,
+            fma(ri, fma(v[0], v[0], mul_(v[1], v[1])),
+                mul_(mul_(v[2], v[2]), k.inv_r)));
+    const double div = fma(dr[0], wx, fma(dr[1], wy, fma(dr[2], wz,
+                           fma(2.0, ri, k.inv_r))));
+    Cons s;
+    s.D = -mul_(c.D, T);
+    const double aa2 = mul_(k.alpha, k.alpha2);
+    // alpha T^ij K_ij
+    const double db = 2.0 * k.alpha2; // d_i beta^j = db alpha^2 D_i l^j + ...
+    const double TK =
+        fma(mul_(lTl, k.c), lH,
+            fma(rl, mul_(db, vH),
+                fma(mul_(rhw, k.c), vA,
+                    mul_(pr.p, fma(mul_(db, k.alpha2), lH,
+                                   mul_(k.c, div))))));
+    s.tau = fma(aa2, fma(-pr.p, vH, mH), fma(-c.tau, T, TK));
+    // momentum: u.d_m l with u = alpha F rhw (v.l) v + c S
+    const double X =
+        fma(aa2, (c.D + c.tau) - pr.p,
+            fma(k.alpha, lTl, mul_(mul_(db, k.alpha2), Sl)));
+    const double q = mul_(mul_(k.alpha, k.F), rl);
+    const double u[3] = {fma(q, v[0], mul_(k.c, c.S[0])),
+                         fma(q, v[1], mul_(k.c, c.S[1])),
+                         fma(q, v[2], mul_(k.c, c.S[2]))};
+    const double wu = fma(u[0], wx, fma(u[1], wy, mul_(u[2], wz)));
+    const double ai = mul_(a, k.inv_ra);
+    const double g[3] = {fma(ri, u[0], -mul_(ai, u[1])),
+                         fma(ri, u[1], mul_(ai, u[0])),
+                         mul_(u[2], k.inv_r)};
+#pragma unroll
+    for (int m = 0; m < 3; ++m)
+        s.S[m] = fma(dH[m], X,
+                     fma(dr[m], wu, fma(-c.S[m], T, g[m])));
+    return s;
+}
+
+// Sum over directions of max |characteristic speed| / dx of a cell with
+// floored primitives (char_speeds, multiplied through by h as face_side).
+GRHD_HD __forceinline__ double ks_inverse_dt(const Options &o,
+                                             const KsCell &k, const Prim &pr,
+                                             const double inv[3])
+{
+    const double vv = ks_vsq(k, pr.v);
+    const double cg = mul_(o.G * (o.G - 1.0), pr.eps); // G p / rho
+    const double h = fma(o.G, pr.eps, 1.0);
+    const double hc = h - cg, den = fma(-vv, cg, h);
+    const double cu = mul_(cg, 1.0 - vv);
+    const double kk = mul_(k.alpha, rcp_ulp(den));
+    double cell = 0.0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+    {
+        const double shift = mul_(k.c, k.l[d]);
+        const double guu = fma(-shift, k.l[d], 1.0);
+        const double vd = pr.v[d];
+        const double base = mul_(vd, hc);
+        const double rad = mul_(cu, fma(guu, den, -mul_(vd, base)));
+        const double root = rad > 0.0 ? mul_(rad, rsqrt_ulp(rad)) : 0.0;
+        const double lo = fma(base - root, kk, -shift);
+        const double hi = fma(base + root, kk, -shift);
+        cell = fma(fmax(fabs(lo), fabs(hi)), inv[d], cell);
+    }
+    return cell;
 }
 
 template <typename A, typename B>

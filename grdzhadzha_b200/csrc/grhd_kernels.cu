@@ -157,6 +157,17 @@ __device__ __forceinline__ bool cell_con2prim(const Options &o, const Cons &c,
     return con2prim_warm(o, c, gUU, p_guess, out);
 }
 
+// The same without a nearby pressure.
+template <typename T>
+__device__ __forceinline__ bool cold_con2prim(const Options &o, const Cons &c,
+                                              const double gUU[6], Prim &out)
+{
+    if constexpr (sizeof(T) == sizeof(double))
+        return con2prim(o, c, gUU, out, nullptr, nullptr);
+    else
+        return con2prim_mixed(o, c, gUU, out, nullptr, nullptr);
+}
+
 template <typename T>
 __device__ __forceinline__ void gLL_double(const GeoT<T> &g, double out[6])
 {
@@ -283,7 +294,7 @@ __device__ __forceinline__ void ghost_at(double *__restrict__ state,
             const Cons sc = load_cons<CG>(state, b.cs,
                                           b.gidx(srcc[0], srcc[1], srcc[2]));
             Prim pr;
-            if (!con2prim(o, sc, sUU, pr, nullptr, nullptr))
+            if (!cold_con2prim<T>(o, sc, sUU, pr))
             {
                 record_error(st, 1, idx);
                 return;
@@ -303,7 +314,7 @@ __device__ __forceinline__ void ghost_at(double *__restrict__ state,
         else
             c = load_cons<CG>(state, b.cs, idx);
         Prim pr;
-        if (!con2prim(o, c, tUU, pr, nullptr, nullptr))
+        if (!cold_con2prim<T>(o, c, tUU, pr))
         {
             record_error(st, 2, idx);
             pr.rho = pr.p = 1.0;
@@ -393,6 +404,49 @@ __device__ __forceinline__ ConsT<T> cell_sources(const Options &o,
     return s;
 }
 
+// Interior cell t of a box (x fastest).  32-bit division, a fifth of the
+// instructions of 64-bit: a box of 2^32 cells would be 378 GB of state.
+__device__ __forceinline__ void interior_cell(const BoxDev &b, int64_t t,
+                                              int &i, int &j, int &k)
+{
+    const unsigned u = (unsigned)t, nx = b.in[0], ny = b.in[1];
+    const unsigned r = u / nx, q = r / ny;
+    i = b.lo[0] + (int)(u - r * nx);
+    j = b.lo[1] + (int)(r - q * ny);
+    k = b.lo[2] + (int)q;
+}
+
+// The per-cell work of the FP64 path on a Kerr-Schild background runs on
+// KsCell (grhd_device.cuh).
+template <typename T, int BGK>
+constexpr bool ks64 = sizeof(T) == sizeof(double) && BGK == 0;
+
+// What the next RHS needs of a cell: con2prim's result `pr` into the
+// primitive cache and the sources of its floored primitives.
+template <typename T>
+__device__ __forceinline__ void
+ks_prep(const Options &o, const Background &bg, const KsCell &kc, double x,
+        double y, double z, bool ok, Prim pr, const Cons &c, T *prim, T *src,
+        const BoxDev &b, int64_t g, int64_t t, DevStatus *st)
+{
+    Cons s = zero_cons<double>();
+    if (!ok)
+    {
+        record_error(st, 2, g);
+        pr.rho = pr.p = 1.0;
+        pr.v[0] = pr.v[1] = pr.v[2] = 0.0;
+        pr.eps = 1.0;
+    }
+    store_pv(prim, b.pcs, g, pr);
+    if (ok && o.use_src)
+    {
+        ks_floors(o, kc, pr);
+        if (!is_atmo(o, pr, o.src_atmo_factor))
+            s = ks_sources(o, bg.a, kc, x, y, z, pr, c);
+    }
+    store_src(src, b.rcs, t, s);
+}
+
 // ------------------------------------------------------- per-cell pass
 
 // Interior cells: con2prim into the primitive cache (the ghosted-box
@@ -400,7 +454,7 @@ __device__ __forceinline__ ConsT<T> cell_sources(const Options &o,
 // k_fill_ghosts) and the sources into the source scratch.  Excised cells
 // keep their frozen primitives and get no source.  The mixed path starts
 // con2prim from the state's stored pressure.
-template <typename T, bool CG = false>
+template <typename T, bool CG = false, int BGK = -1>
 __device__ __forceinline__ void cells_item(const double *__restrict__ state,
                                            T *__restrict__ prim,
                                            T *__restrict__ src,
@@ -410,10 +464,8 @@ __device__ __forceinline__ void cells_item(const double *__restrict__ state,
                                            int64_t t)
 {
     {
-        const int i = b.lo[0] + (int)(t % b.in[0]);
-        const int64_t r = t / b.in[0];
-        const int j = b.lo[1] + (int)(r % b.in[1]);
-        const int k = b.lo[2] + (int)(r / b.in[1]);
+        int i, j, k;
+        interior_cell(b, t, i, j, k);
         const int64_t g = b.gidx(i, j, k);
         ConsT<T> s = zero_cons<T>();
         if (excised(o, i, j, k))
@@ -424,11 +476,21 @@ __device__ __forceinline__ void cells_item(const double *__restrict__ state,
         }
         double x, y, z;
         cell_xyz(o, i, j, k, x, y, z);
+        if constexpr (ks64<T, BGK>)
+        {
+            const Cons c = load_cons<CG>(state, b.cs, g);
+            KsCell kc;
+            ks_cell(bg.M, bg.a, x, y, z, kc);
+            Prim pr;
+            const bool ok = ks_con2prim(o, kc, c, pr);
+            ks_prep(o, bg, kc, x, y, z, ok, pr, c, prim, src, b, g, t, st);
+            return;
+        }
         GeoFullT<T> f;
         if (o.use_src)
-            metric_T<T, true>(bg, x, y, z, f.g, &f);
+            metric_T<T, true, BGK>(bg, x, y, z, f.g, &f);
         else
-            metric_T<T, false>(bg, x, y, z, f.g, nullptr);
+            metric_T<T, false, BGK>(bg, x, y, z, f.g, nullptr);
         const Cons c = load_cons<CG>(state, b.cs, g);
         Prim pr;
         if (!cell_con2prim(o, c, f.g, rd<CG>(&state[kPress * b.cs + g]), pr))
@@ -445,7 +507,7 @@ __device__ __forceinline__ void cells_item(const double *__restrict__ state,
     }
 }
 
-template <typename T>
+template <typename T, int BGK>
 __global__ void __launch_bounds__(256, kMinBlocks<T>)
     k_cells(const double *__restrict__ state, T *__restrict__ prim,
             T *__restrict__ src, BoxDev b, Background bg, Options o,
@@ -454,7 +516,7 @@ __global__ void __launch_bounds__(256, kMinBlocks<T>)
     const int64_t n = b.ivol();
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
          t += (int64_t)gridDim.x * blockDim.x)
-        cells_item<T>(state, prim, src, b, bg, o, st, t);
+        cells_item<T, false, BGK>(state, prim, src, b, bg, o, st, t);
 }
 
 // ----------------------------------------------------------- face pass
@@ -958,15 +1020,6 @@ __device__ __forceinline__ void flush_counts(DevStatus *st,
     }
 }
 
-__device__ __forceinline__ void interior_cell(const BoxDev &b, int64_t t,
-                                              int &i, int &j, int &k)
-{
-    i = b.lo[0] + (int)(t % b.in[0]);
-    const int64_t r = t / b.in[0];
-    j = b.lo[1] + (int)(r % b.in[1]);
-    k = b.lo[2] + (int)(r / b.in[1]);
-}
-
 // update_conserved: dst = src + dt * rhs on the interior
 // (add_scaled_conserved_rhs, FArrayBoxFiniteVolume.hpp:927-940), then the
 // post-update recovery when `recover` is set.
@@ -1194,6 +1247,59 @@ stage_item(const double *un, int64_t ucs, const double *us, int64_t tcs,
         c.tau = u[4];
         double x, y, z;
         cell_xyz(o, i, j, k, x, y, z);
+        if constexpr (ks64<T, BGK>)
+        {
+            KsCell kc;
+            ks_cell(bg.M, bg.a, x, y, z, kc);
+            // recovery with atmosphere (:60-110)
+            Prim pr, stored;
+            bool ok = ks_con2prim(o, kc, c, pr);
+            bool reset = !ok;
+            cnt[0] += 1;
+            if (ok)
+            {
+                stored = pr;
+                ks_floors(o, kc, stored);
+                reset = primitive_differs(pr, stored);
+                if (reset)
+                    cnt[2] += 1;
+            }
+            else
+            {
+                cnt[1] += 1;
+                stored = atmosphere(o);
+            }
+            if (store_p)
+                store_prim(out, ocs, g, stored);
+            if (reset)
+            {
+                cnt[3] += 1;
+                double gLL[6];
+                ks_gLL(kc, gLL);
+                c = p2c(stored, gLL);
+            }
+            store_cons(out, ocs, g, c);
+            if (prep || cfl)
+            {
+                // con2prim of the state just written (an unchanged cell's
+                // is pr)
+                if (reset)
+                    ok = ks_con2prim(o, kc, c, pr);
+                if (!ok && !prep)
+                    record_error(st, 4, b.t0 + t);
+                if (cfl && ok)
+                {
+                    Prim fp = pr;
+                    ks_floors(o, kc, fp);
+                    if (!is_atmo(o, fp, 1.0 + 1.0e-12))
+                        cell_inv = ks_inverse_dt(o, kc, fp, inv);
+                }
+                if (prep)
+                    ks_prep(o, bg, kc, x, y, z, ok, pr, c, prim, src, b, g, t,
+                            st);
+            }
+            return;
+        }
         GeoFullT<T> f;
         if (prep && o.use_src)
             metric_T<T, true, BGK>(bg, x, y, z, f.g, &f);
@@ -1338,8 +1444,8 @@ __device__ __forceinline__ double cfl_item(const double *__restrict__ state,
         for (int q = 0; q < 6; ++q)
             gUU[q] = double(geo.gUU[q]);
         Prim pr;
-        if (!con2prim(o, load_cons<CG>(state, b.cs, b.gidx(i, j, k)), gUU, pr,
-                      nullptr, nullptr))
+        if (!cold_con2prim<T>(
+                o, load_cons<CG>(state, b.cs, b.gidx(i, j, k)), gUU, pr))
             record_error(st, 4, b.t0 + t);
         else
             cell = cfl_speed<T>(o, pr, geo, inv);
@@ -1570,6 +1676,10 @@ __device__ __forceinline__ double ens_dt(const EnsMember &m,
     return dt;
 }
 
+// Members are Kerr-Schild boxes; the FP32 arithmetic measured no faster
+// with the kind fixed at compile time and keeps its code.
+template <typename T> constexpr int kEnsBgk = sizeof(T) == 8 ? 0 : -1;
+
 template <typename T>
 __device__ __forceinline__ const FaceOpt<T> &
 member_face_opt(const EnsMember &m)
@@ -1659,7 +1769,7 @@ __global__ void __launch_bounds__(kEnsItemCells, kMinBlocks<T>)
                 const int64_t t =
                     (it - __ldg(&a.off_cell[m])) * kEnsItemCells + tid;
                 if (t < ms.b.ivol())
-                    cells_item<T, true>(ms.state, static_cast<T *>(ms.prim),
+                    cells_item<T, true, kEnsBgk<T>>(ms.state, static_cast<T *>(ms.prim),
                                         static_cast<T *>(ms.src), ms.b, ms.bg,
                                         ms.o, ms.st, t);
             }
@@ -1760,7 +1870,7 @@ __global__ void __launch_bounds__(kEnsItemCells, kMinBlocks<T>)
                     unsigned long long cnt[4] = {0ull, 0ull, 0ull, 0ull};
                     double ci = 0.0;
                     if (t < ms.b.ivol())
-                        stage_item<0, T, true>(
+                        stage_item<0, T, true, kEnsBgk<T>>(
                             ms.state, ms.b.cs, nullptr, 0,
                             s < 3 ? ms.stage : ms.state,
                             s < 3 ? ms.sb.cs : ms.b.cs,
@@ -1913,10 +2023,11 @@ __device__ __forceinline__ Geo geo_get(const double *__restrict__ gc,
 __device__ __forceinline__ void ghosted_cell(const BoxDev &b, int64_t t,
                                              int &i, int &j, int &k)
 {
-    i = b.glo[0] + (int)(t % b.gn[0]);
-    const int64_t r = t / b.gn[0];
-    j = b.glo[1] + (int)(r % b.gn[1]);
-    k = b.glo[2] + (int)(r / b.gn[1]);
+    const unsigned u = (unsigned)t, nx = b.gn[0], ny = b.gn[1];
+    const unsigned r = u / nx, q = r / ny;
+    i = b.glo[0] + (int)(u - r * nx);
+    j = b.glo[1] + (int)(r - q * ny);
+    k = b.glo[2] + (int)q;
 }
 
 // fill_conserved_outflow_boundaries (:484-519) and
@@ -2449,8 +2560,16 @@ void launch_cells(const double *state, T *prim, T *src, const BoxDev &b,
                   const Background &bg, const Options &o, DevStatus *st,
                   cudaStream_t s)
 {
-    k_cells<T><<<grid_for(b.ivol(), 256), 256, 0, s>>>(state, prim, src, b, bg,
-                                                       o, st);
+    // (the mixed path keeps the run-time background: its results stay as they
+    // are)
+    auto go = [&](auto kern) {
+        kern<<<grid_for(b.ivol(), 256), 256, 0, s>>>(state, prim, src, b, bg,
+                                                     o, st);
+    };
+    if (sizeof(T) == sizeof(float))
+        go(k_cells<T, -1>);
+    else
+        bg.kind == 1 ? go(k_cells<T, 1>) : go(k_cells<T, 0>);
 }
 
 template <typename T>
