@@ -577,7 +577,17 @@ __device__ __forceinline__ void background_metric_mixed(const Background &bg,
     if (BGK == 1 || (BGK < 0 && bg.kind == 1))
         pn_metric<float, FULL>(bg, float(x), float(y), float(z), g, f);
     else if (x * x + y * y + z * z < 9.0 * bg.M * bg.M)
-        ks_metric_fp64_to_fp32<FULL>(bg.M, bg.a, x, y, z, g, f);
+    {
+        // through temporaries: the call's results live in local memory, and
+        // the caller's fields would too, on every path, if it got their
+        // address
+        GeoT<float> gt;
+        GeoFullT<float> ft;
+        ks_metric_fp64_to_fp32<FULL>(bg.M, bg.a, x, y, z, gt, &ft);
+        g = gt;
+        if (FULL)
+            *f = ft;
+    }
     else
         ks_metric<float, FULL>(float(bg.M), float(bg.a), float(x), float(y),
                                float(z), g, f);
@@ -949,36 +959,33 @@ GRHD_HD __forceinline__ bool con2prim_warm(const Options &o, const Cons &c,
                                               const double gUU[6],
                                               double p_guess, Prim &out)
 {
-    if (c.D > 0.0 && !(p_guess > o.rec_pfloor))
+    if (c.D > 0.0)
     {
+        const double Gfac = div_(o.G, o.G - 1.0);
+        const double tD = c.tau + c.D;
+        double mU[3];
+        raise(gUU, c.S, mU);
+        const double S2 = dot3(c.S, mU);
         // a guess at (or rounded below) the recovery floor: the full solve
         // returns the floor itself when the residual there is within
-        // tolerance; test that first
-        const double G = o.G;
-        const double S2 = c2p_S2(c, gUU);
-        const double r = c2p_residual(o.rec_pfloor, c.D, c.tau, S2, G,
-                                      div_(G, G - 1.0), o.rec_vmax2, nullptr);
-        if (fabs(r) <= o.rec_tol)
-            return c2p_finish_gUU(o, c, gUU, S2, o.rec_pfloor, out) ||
-                   con2prim_mixed(o, c, gUU, out, nullptr, nullptr);
-    }
-    if (c.D > 0.0 && p_guess > o.rec_pfloor && isfinite(p_guess))
-    {
-        const double G = o.G;
-        const double Gfac = div_(G, G - 1.0);
-        const double S2 = c2p_S2(c, gUU);
-        double p = p_guess, dres;
-        double r = c2p_residual(p, c.D, c.tau, S2, G, Gfac, o.rec_vmax2, &dres);
-        for (int it = 0; it < 6; ++it)
+        // tolerance; only that is tested
+        const bool at_floor = !(p_guess > o.rec_pfloor);
+        if (at_floor || isfinite(p_guess))
         {
-            if (fabs(r) < o.rec_tol)
-                return c2p_finish_gUU(o, c, gUU, S2, p, out) ||
-                       con2prim_mixed(o, c, gUU, out, nullptr, nullptr);
-            const double np = p - div_(r, dres);
-            if (!isfinite(np) || !(np > o.rec_pfloor))
-                break;
-            p = np;
-            r = c2p_residual(p, c.D, c.tau, S2, G, Gfac, o.rec_vmax2, &dres);
+            double p = at_floor ? o.rec_pfloor : p_guess, dres;
+            double r = c2p_f(p, c.D, tD, S2, Gfac, o.rec_vmax2, dres);
+            bool found =
+                at_floor ? fabs(r) <= o.rec_tol : fabs(r) < o.rec_tol;
+            for (int it = 1; !at_floor && !found && it < 6; ++it)
+            {
+                p = fma(-r, rcp_ulp(dres), p);
+                if (!isfinite(p) || !(p > o.rec_pfloor))
+                    break;
+                r = c2p_f(p, c.D, tD, S2, Gfac, o.rec_vmax2, dres);
+                found = fabs(r) < o.rec_tol;
+            }
+            if (found && c2p_finish(o, c, mU, S2, p, out))
+                return true;
         }
     }
     return con2prim_mixed(o, c, gUU, out, nullptr, nullptr);

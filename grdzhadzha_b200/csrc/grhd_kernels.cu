@@ -46,6 +46,15 @@ __device__ __forceinline__ void record_error(DevStatus *st, int where,
 // tile's 108 KB of shared memory allows no more).
 template <typename T> constexpr int kMinBlocks = sizeof(T) == 4 ? 3 : 2;
 
+// The stage kernel's blocks: where its state fits 80 registers with few
+// spills, a third block hides more latency than they cost (ms per launch:
+// FP64 Kerr-Schild at 256^3 1.36 with three, 1.53 with two; mixed binary at
+// 320^3 3.2 and 3.9); the other two keep two (mixed Kerr-Schild at 256^3
+// 1.49 with two, 1.63 with three; FP64 binary at 128^3 0.24 and 0.26).
+constexpr int kStageThreads = 256;
+template <typename T, int BGK>
+constexpr int kStageBlocks = (sizeof(T) == 8) == (BGK == 0) ? 3 : 2;
+
 // Loads of data that a persistent launch wrote itself in an earlier phase
 // (CG = true) go through L2 (ld.global.cg): the non-coherent read-only path
 // (__ldg) is only valid for data left unchanged for a whole launch.
@@ -508,7 +517,7 @@ __device__ __forceinline__ void cells_item(const double *__restrict__ state,
 }
 
 template <typename T, int BGK>
-__global__ void __launch_bounds__(256, kMinBlocks<T>)
+__global__ void __launch_bounds__(256, 3)
     k_cells(const double *__restrict__ state, T *__restrict__ prim,
             T *__restrict__ src, BoxDev b, Background bg, Options o,
             DevStatus *st)
@@ -1184,23 +1193,52 @@ __device__ __forceinline__ void flush_max(DevStatus *st, double v)
 // 942-969).  The stage input k, the primitive cache and the sources are of
 // type T; U, the accumulator and con2prim are FP64.  The mixed path starts
 // con2prim from the primitive cache's pressure of the same cell.
+// What a stage reads of one cell: U^n, the stage input k, a second vector v
+// (the accumulator after RK4's first stage, U^1 in mode 2) and the mixed
+// path's starting pressure.
+template <typename T> struct StageIn
+{
+    double u[5], v[5];
+    T k[5], p;
+};
+
+static_assert(kD == 0 && kS1 == 1 && kTau == 4,
+              "the conserved components come first, in the RHS's order");
+
+template <int MODE, typename T, bool CG>
+__device__ __forceinline__ void
+stage_load(StageIn<T> &in, const double *un, int64_t ucs, const double *us,
+           int64_t tcs, const T *__restrict__ kv,
+           const double *__restrict__ acc, const T *__restrict__ prim_in,
+           const BoxDev &b, int stage, int64_t g, int64_t t)
+{
+#pragma unroll
+    for (int c = 0; c < 5; ++c)
+    {
+        in.u[c] = rd<CG>(&un[c * ucs + g]);
+        in.k[c] = rd<CG>(&kv[c * b.rcs + t]);
+        if (MODE == 0 && stage > 0)
+            in.v[c] = rd<CG>(&acc[c * b.rcs + t]);
+        if (MODE == 2)
+            in.v[c] = rd<CG>(&us[c * tcs + g]);
+    }
+    if (sizeof(T) != sizeof(double))
+        in.p = prim_in ? rd<CG>(&prim_in[1 * b.pcs + g]) : T(0);
+}
+
 template <int MODE, typename T, bool CG = false, int BGK = -1>
 __device__ __forceinline__ void
-stage_item(const double *un, int64_t ucs, const double *us, int64_t tcs,
-           double *out, int64_t ocs, const T *__restrict__ kv,
-           double *__restrict__ acc, T *__restrict__ prim,
+stage_item(const StageIn<T> &in, const double *un, int64_t ucs, double *out,
+           int64_t ocs, double *__restrict__ acc, T *__restrict__ prim,
            T *__restrict__ src, const BoxDev &b, const Background &bg,
            const Options &o, int stage, double dt, bool prep, bool store_p,
-           bool cfl, const double inv[3], DevStatus *st, int64_t t,
-           unsigned long long cnt[4], double &cell_inv,
-           const T *__restrict__ prim_in = nullptr)
+           bool cfl, const double inv[3], DevStatus *st, int64_t t, int i,
+           int j, int k, int64_t g, unsigned long long cnt[4],
+           double &cell_inv)
 {
     const double cst = (stage == 2) ? dt : 0.5 * dt;
     const double dt6 = dt / 6.0;
     const bool mixed = sizeof(T) != sizeof(double);
-    int i, j, k;
-    interior_cell(b, t, i, j, k);
-    const int64_t g = b.gidx(i, j, k);
     if (excised(o, i, j, k))
     {
         if (out != un)
@@ -1214,16 +1252,15 @@ stage_item(const double *un, int64_t ucs, const double *us, int64_t tcs,
     }
     else
     {
-        const int comp_of[5] = {kD, kS1, kS1 + 1, kS1 + 2, kTau};
         double u[5];
 #pragma unroll
         for (int c = 0; c < 5; ++c)
         {
-            const double kk = double(rd<CG>(&kv[c * b.rcs + t]));
-            const double u0 = rd<CG>(&un[comp_of[c] * ucs + g]);
+            const double kk = double(in.k[c]);
+            const double u0 = in.u[c];
             if (MODE == 0)
             {
-                double a = (stage == 0) ? kk : rd<CG>(&acc[c * b.rcs + t]);
+                double a = (stage == 0) ? kk : in.v[c];
                 if (stage == 1 || stage == 2)
                     a = a + 2.0 * kk;
                 if (stage < 3)
@@ -1237,7 +1274,7 @@ stage_item(const double *un, int64_t ucs, const double *us, int64_t tcs,
             else if (MODE == 1)
                 u[c] = u0 + dt * kk;
             else
-                u[c] = 0.5 * (u0 + rd<CG>(&us[comp_of[c] * tcs + g]) + dt * kk);
+                u[c] = 0.5 * (u0 + in.v[c] + dt * kk);
         }
         Cons c;
         c.D = u[0];
@@ -1307,9 +1344,7 @@ stage_item(const double *un, int64_t ucs, const double *us, int64_t tcs,
             metric_T<T, false, BGK>(bg, x, y, z, f.g, nullptr);
         double gLL[6];
         gLL_double(f.g, gLL);
-        const T *pg = prim_in ? prim_in : prim;
-        const double p_guess =
-            (mixed && pg) ? double(rd<CG>(&pg[1 * b.pcs + g])) : 0.0;
+        const double p_guess = mixed ? double(in.p) : 0.0;
         // recovery with atmosphere (:60-110)
         Prim pr;
         const bool ok = cell_con2prim(o, c, f.g, p_guess, pr);
@@ -1385,7 +1420,7 @@ stage_item(const double *un, int64_t ucs, const double *us, int64_t tcs,
 }
 
 template <int MODE, typename T, int BGK>
-__global__ void __launch_bounds__(256, kMinBlocks<T>)
+__global__ void __launch_bounds__(kStageThreads, kStageBlocks<T, BGK>)
     k_stage(const double *un, int64_t ucs, const double *us, int64_t tcs,
             double *out, int64_t ocs, const T *__restrict__ kv,
             double *__restrict__ acc, T *__restrict__ prim,
@@ -1393,6 +1428,32 @@ __global__ void __launch_bounds__(256, kMinBlocks<T>)
             int stage, double dt, int prep_flag, int cfl, double i0,
             double i1, double i2, DevStatus *st, const T *__restrict__ prim_in)
 {
+    // Each thread's inputs of its next cell arrive in its own shared-memory
+    // slots (asynchronous copies) while it works on the current one: the
+    // kernel's loads were half of its stalls.  Per launch at 256^3, FP64
+    // 1.53 -> 1.20 ms and mixed 1.73 -> 1.45 (the bytes alone take 0.72 and
+    // 0.58), mixed binary at 320^3 3.40 -> 3.04.
+    constexpr bool mixed = sizeof(T) != sizeof(double);
+    __shared__ double sd[10][kStageThreads];
+    __shared__ T sk[mixed ? 6 : 5][kStageThreads];
+    const int tid = threadIdx.x;
+    const T *pg = prim_in ? prim_in : prim;
+    const bool want_v = MODE == 2 || (MODE == 0 && stage > 0);
+    auto fetch = [&](int64_t g, int64_t t) {
+#pragma unroll
+        for (int c = 0; c < 5; ++c)
+        {
+            cp_async_elem(&sd[c][tid], &un[c * ucs + g]);
+            cp_async_elem(&sk[c][tid], &kv[c * b.rcs + t]);
+            if (MODE == 0 && stage > 0)
+                cp_async_elem(&sd[5 + c][tid], &acc[c * b.rcs + t]);
+            if (MODE == 2)
+                cp_async_elem(&sd[5 + c][tid], &us[c * tcs + g]);
+        }
+        if constexpr (mixed)
+            if (pg)
+                cp_async_elem(&sk[5][tid], &pg[1 * b.pcs + g]);
+    };
     unsigned long long cnt[4] = {0, 0, 0, 0};
     const int64_t n = b.ivol();
     const int64_t n_pad = (n + blockDim.x - 1) / blockDim.x * blockDim.x;
@@ -1401,15 +1462,45 @@ __global__ void __launch_bounds__(256, kMinBlocks<T>)
     // keeps its primitives even so (the last RK4 stage of a multi-step call)
     const bool prep = (prep_flag & 1) && prim != nullptr;
     const bool store_p = !prep || (prep_flag & 2);
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n_pad;
-         t += (int64_t)gridDim.x * blockDim.x)
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    int64_t t = blockIdx.x * (int64_t)blockDim.x + tid;
+    int i, j, k;
+    int64_t g = 0;
+    if (t < n)
+    {
+        interior_cell(b, t, i, j, k);
+        g = b.gidx(i, j, k);
+        fetch(g, t);
+    }
+    for (; t < n_pad; t += step)
     {
         double cell_inv = 0.0;
         if (t < n)
-            stage_item<MODE, T, false, BGK>(un, ucs, us, tcs, out, ocs, kv, acc,
-                                            prim, src,
-                                b, bg, o, stage, dt, prep, store_p, cfl != 0,
-                                inv, st, t, cnt, cell_inv, prim_in);
+        {
+            const int ci = i, cj = j, ck = k;
+            const int64_t cg = g;
+            StageIn<T> in;
+            cp_async_wait_all();
+#pragma unroll
+            for (int c = 0; c < 5; ++c)
+            {
+                in.u[c] = sd[c][tid];
+                in.k[c] = sk[c][tid];
+                in.v[c] = want_v ? sd[5 + c][tid] : 0.0;
+            }
+            if constexpr (mixed)
+                in.p = pg ? sk[5][tid] : T(0);
+            if (t + step < n)
+            {
+                interior_cell(b, t + step, i, j, k);
+                g = b.gidx(i, j, k);
+                fetch(g, t + step);
+            }
+            stage_item<MODE, T, false, BGK>(
+                in, un, ucs, out, ocs, acc, prim, src, b, bg, o, stage, dt,
+                prep, store_p, cfl != 0, inv, st, t, ci, cj, ck, cg, cnt,
+                cell_inv);
+        }
         flush_counts(st, cnt);
         cnt[0] = cnt[1] = cnt[2] = cnt[3] = 0;
         if (cfl)
@@ -1870,15 +1961,23 @@ __global__ void __launch_bounds__(kEnsItemCells, kMinBlocks<T>)
                     unsigned long long cnt[4] = {0ull, 0ull, 0ull, 0ull};
                     double ci = 0.0;
                     if (t < ms.b.ivol())
-                        stage_item<0, T, true, kEnsBgk<T>>(
-                            ms.state, ms.b.cs, nullptr, 0,
-                            s < 3 ? ms.stage : ms.state,
-                            s < 3 ? ms.sb.cs : ms.b.cs,
+                    {
+                        int ic, jc, kc;
+                        interior_cell(ms.b, t, ic, jc, kc);
+                        const int64_t g = ms.b.gidx(ic, jc, kc);
+                        StageIn<T> in;
+                        stage_load<0, T, true>(
+                            in, ms.state, ms.b.cs, nullptr, 0,
                             static_cast<const T *>(ms.k), ms.acc,
+                            static_cast<const T *>(ms.prim), ms.b, s, g, t);
+                        stage_item<0, T, true, kEnsBgk<T>>(
+                            in, ms.state, ms.b.cs, s < 3 ? ms.stage : ms.state,
+                            s < 3 ? ms.sb.cs : ms.b.cs, ms.acc,
                             static_cast<T *>(ms.prim),
                             static_cast<T *>(ms.src), ms.b, ms.bg, ms.o, s,
-                            dt, true, s == 3, s == 3, ms.inv, ms.st, t, cnt,
-                            ci);
+                            dt, true, s == 3, s == 3, ms.inv, ms.st, t, ic,
+                            jc, kc, g, cnt, ci);
+                    }
                     flush_counts(ms.st, cnt);
                     if (s == 3)
                         flush_max_to(&ms.mi_bits[(step + 1ull) & 1ull], ci);
@@ -2617,6 +2716,18 @@ void launch_recover(double *state, const BoxDev &b, const Background &bg,
     k_recover<<<grid_for(b.ivol(), 256), 256, 0, s>>>(state, b, bg, o, st);
 }
 
+// Blocks of a stage launch: two cells a thread where that leaves four waves
+// of blocks, so that a thread's second cell arrives during its first.  More
+// cells a thread lose to the spread of their costs (fluid, atmosphere,
+// excised): at 256^3 FP64 1.20 ms with two, 1.38 with 14, 1.80 with one wave
+// of blocks; at 64^3, two cells in 1.2 waves take 32 us against 28 with one.
+template <typename T> int stage_grid(int64_t n, int kind)
+{
+    const int64_t blocks = (n + kStageThreads - 1) / kStageThreads;
+    const int per = kind == 1 ? kStageBlocks<T, 1> : kStageBlocks<T, 0>;
+    return (int)(blocks >= 8 * 148 * per ? (blocks + 1) / 2 : blocks);
+}
+
 template <typename T>
 void launch_stage(int mode, const double *un, int64_t ucs, const double *us,
                   int64_t tcs, double *out, int64_t ocs, const T *k,
@@ -2625,12 +2736,12 @@ void launch_stage(int mode, const double *un, int64_t ucs, const double *us,
                   double dt, bool cfl, const double inv_dx[3], DevStatus *st,
                   cudaStream_t s, const T *prim_in)
 {
-    const int grid = grid_for(b.ivol(), 256);
+    const int grid = stage_grid<T>(b.ivol(), bg.kind);
     const double i0 = inv_dx ? inv_dx[0] : 0.0, i1 = inv_dx ? inv_dx[1] : 0.0,
                  i2 = inv_dx ? inv_dx[2] : 0.0;
     const int pf = prep, cf = cfl ? 1 : 0;
     auto go = [&](auto kern) {
-        kern<<<grid, 256, 0, s>>>(un, ucs, us, tcs, out, ocs, k, acc, prim, src,
+        kern<<<grid, kStageThreads, 0, s>>>(un, ucs, us, tcs, out, ocs, k, acc, prim, src,
                                   b, bg, o, stage, dt, pf, cf, i0, i1, i2, st,
                                   prim_in);
     };
