@@ -2249,6 +2249,7 @@ int grhd_level_exchange_components(const grhd_box *boxes,
                                 GRHD_ERR_INVALID_ARG);
         }
     cudaStream_t s = (cudaStream_t)stream;
+    std::vector<CopyRegion> regions;
     for (int a = 0; a < count; ++a)
         for (int q = 0; q < count; ++q)
         {
@@ -2267,9 +2268,10 @@ int grhd_level_exchange_components(const grhd_box *boxes,
                 any = any && lo[d] <= hi[d];
             }
             if (any)
-                launch_copy_region(states[a], b[a], states[q], b[q], lo, hi,
-                                   ncomp, s);
+                regions.push_back(copy_region(states[a], b[a], states[q],
+                                              b[q], lo, hi));
         }
+    launch_copy_regions(regions.data(), regions.size(), ncomp, s);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return io_error(err, err_cap, cudaGetErrorString(e), GRHD_ERR_CUDA);

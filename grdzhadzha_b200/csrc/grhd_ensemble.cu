@@ -110,6 +110,36 @@ void member_tiles(const BoxDev &b, int zchunk, int t[3])
     t[2] = (b.in[2] + zchunk - 1) / zchunk;
 }
 
+// The launch shape until the autotuner or the caller sets another: every
+// block that fits, since the phases wait on latency (24 mixed members of
+// 32..96 cells a side, two steps: 50.4 ms with one block per SM, 23.8 with
+// three), and of 32, 16, 8 and 4 planes a face tile the count whose tiles
+// fill the fewest waves of blocks (a tile costs its planes and 0.7 of one;
+// five members of 32..48: 4.9 ms with 32 planes, 1.5 with 4).
+grhd_ensemble_tuning default_tuning(const grhd_ensemble *e)
+{
+    grhd_ensemble_tuning best = {32, e->max_bps, 0.0};
+    const int64_t slots = (int64_t)e->max_bps * e->num_sms;
+    double best_cost = 0.0;
+    for (int z : {32, 16, 8, 4})
+    {
+        int64_t tiles = 0;
+        for (const EnsMember &d : e->desc)
+        {
+            int t[3];
+            member_tiles(d.b, z, t);
+            tiles += (int64_t)t[0] * t[1] * t[2];
+        }
+        const double cost = (z + 0.7) * (double)((tiles + slots - 1) / slots);
+        if (best_cost == 0.0 || cost < best_cost)
+        {
+            best_cost = cost;
+            best.zchunk = z;
+        }
+    }
+    return best;
+}
+
 // Fills the tiling fields of the descriptors and the prefix tables for the
 // current tuning and uploads both.
 int upload_layout(grhd_ensemble *e)
@@ -314,7 +344,6 @@ int build(grhd_ensemble *e)
         return ens_error(e, GRHD_ERR_CUDA,
                          "the ensemble kernel does not fit on an SM");
     e->max_bps = bps;
-    e->tuning.blocks_per_sm = 1;
 
     // scratch arena
     std::vector<size_t> base(n);
@@ -391,6 +420,7 @@ int build(grhd_ensemble *e)
     e->ctl_h->need_cfl = 1;
     ENS_CUDA(e, cudaMemcpy(e->ctl, e->ctl_h, sizeof(EnsControl),
                            cudaMemcpyHostToDevice));
+    e->tuning = default_tuning(e);
     return upload_layout(e);
 }
 

@@ -32,12 +32,30 @@ void launch_state_to_checkpoint(const double *state, const BoxDev &b,
 void launch_checkpoint_to_state(const double *in, const BoxDev &b, int ncomp,
                                 double *state, cudaStream_t s);
 
-// LevelData::exchange between two boxes of a level: the first `ncomp`
-// components of the cells [lo, hi] (level index space) from `src` (box sb)
-// to `dst` (box db).
-void launch_copy_region(double *dst, const BoxDev &db, const double *src,
-                        const BoxDev &sb, const int lo[3], const int hi[3],
-                        int ncomp, cudaStream_t s);
+// One region of LevelData::exchange: the cells [lo, hi] (level index space)
+// of `dst` (box db) from `src` (box sb), as pointers to the first cell and
+// strides.
+struct CopyRegion
+{
+    double *dst;
+    const double *src;
+    int64_t dst_cs, src_cs, dst_plane, src_plane;
+    int dst_row, src_row, n[3];
+};
+// The regions of one launch, passed by value (the kernel arguments' 4 KB).
+struct CopyBatch
+{
+    static constexpr int kMax = 48;
+    CopyRegion r[kMax];
+};
+static_assert(sizeof(CopyBatch) <= 4000, "fits the kernel arguments");
+
+CopyRegion copy_region(double *dst, const BoxDev &db, const double *src,
+                       const BoxDev &sb, const int lo[3], const int hi[3]);
+// Copies the first `ncomp` components of all regions (no region's source is
+// another's destination).
+void launch_copy_regions(const CopyRegion *r, size_t count, int ncomp,
+                         cudaStream_t s);
 
 // The first `ncomp` components of the region [lo, hi] (inside the ghosted
 // box) into (pack) or out of a packed buffer [component][k][j][i].
