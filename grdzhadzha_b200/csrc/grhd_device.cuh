@@ -961,11 +961,9 @@ GRHD_HD __forceinline__ bool con2prim_warm(const Options &o, const Cons &c,
 {
     if (c.D > 0.0)
     {
-        const double Gfac = div_(o.G, o.G - 1.0);
-        const double tD = c.tau + c.D;
-        double mU[3];
-        raise(gUU, c.S, mU);
-        const double S2 = dot3(c.S, mU);
+        const double G = o.G;
+        const double Gfac = div_(G, G - 1.0);
+        const double S2 = c2p_S2(c, gUU);
         // a guess at (or rounded below) the recovery floor: the full solve
         // returns the floor itself when the residual there is within
         // tolerance; only that is tested
@@ -973,18 +971,20 @@ GRHD_HD __forceinline__ bool con2prim_warm(const Options &o, const Cons &c,
         if (at_floor || isfinite(p_guess))
         {
             double p = at_floor ? o.rec_pfloor : p_guess, dres;
-            double r = c2p_f(p, c.D, tD, S2, Gfac, o.rec_vmax2, dres);
+            double r =
+                c2p_residual(p, c.D, c.tau, S2, G, Gfac, o.rec_vmax2, &dres);
             bool found =
                 at_floor ? fabs(r) <= o.rec_tol : fabs(r) < o.rec_tol;
             for (int it = 1; !at_floor && !found && it < 6; ++it)
             {
-                p = fma(-r, rcp_ulp(dres), p);
+                p = p - div_(r, dres);
                 if (!isfinite(p) || !(p > o.rec_pfloor))
                     break;
-                r = c2p_f(p, c.D, tD, S2, Gfac, o.rec_vmax2, dres);
+                r = c2p_residual(p, c.D, c.tau, S2, G, Gfac, o.rec_vmax2,
+                                 &dres);
                 found = fabs(r) < o.rec_tol;
             }
-            if (found && c2p_finish(o, c, mU, S2, p, out))
+            if (found && c2p_finish_gUU(o, c, gUU, S2, p, out))
                 return true;
         }
     }
