@@ -660,7 +660,8 @@ int grhd_recover_primitives(grhd_ctx *ctx, double *state, int64_t state_cs,
     const Background bg = make_background(ctx->params, time);
     {
         Timed t_(ctx, GRHD_K_STAGE, s);
-        launch_recover(state, b, bg, ctx->opt, ctx->status, s);
+        launch_recover(state, b, bg, ctx->opt, ctx->status,
+                       ctx->params.precision == GRHD_PRECISION_MIXED, s);
     }
     st = finish_status(ctx, b, state, bg, s);
     read_diag(ctx, diag);
@@ -689,7 +690,8 @@ int grhd_update_conserved(grhd_ctx *ctx, double *state, int64_t state_cs,
     {
         Timed t_(ctx, GRHD_K_STAGE, s);
         launch_update(state, b.cs, state, b.cs, rhs, b, bg, ctx->opt, dt,
-                      recover, ctx->status, s);
+                      recover, ctx->status,
+                      ctx->params.precision == GRHD_PRECISION_MIXED, s);
     }
     st = finish_status(ctx, b, state, bg, s);
     read_diag(ctx, diag);
@@ -2051,7 +2053,7 @@ int grhd_kitp_advance_ssprk2(grhd_ctx *ctx, double *state, int64_t state_cs,
     launch_kitp_combine(state, b, ctx->stage, sb.cs, k, b.ivol(), dt, s);
     if (cfg->sink_rate != 0.0 && cfg->sink_size > 0.0)
         launch_kitp_sink_decay(state, b, ctx->opt, kh, dt, s);
-    launch_recover(state, b, bg1, ctx->opt, ctx->status, s);
+    launch_recover(state, b, bg1, ctx->opt, ctx->status, false, s);
     ctx->launches += 4 + (visc ? 2 : 0);
     st = finish_status(ctx, b, state, bg0, s);
     read_diag(ctx, diag);

@@ -377,6 +377,75 @@ GRHD_HD __forceinline__ void ks_metric(T M, T a, T x, T y, T z,
     f->g = g;
 }
 
+// An FP64 Kerr-Schild cell in terms of its null vector l and H (see "FP64
+// Kerr-Schild cell" below).
+struct KsCell
+{
+    double l[3], F, c, alpha, alpha2;
+    double r, inv_r, inv_ra, inv_sigma; // 1/r, 1/(r^2 + a^2), 1/Sigma
+};
+
+GRHD_HD __forceinline__ void ks_cell(double M, double a, double x, double y,
+                                     double z, KsCell &k)
+{
+    const double a2 = mul_(a, a);
+    const double rho2 =
+        fmax(fma(x, x, fma(y, y, mul_(z, z))), 1.0e-12); // (1e-6)^2
+    const double hA = 0.5 * (rho2 - a2);
+    const double az = mul_(a, z);
+    const double r2 = hA + sqrt_(fma(hA, hA, mul_(az, az)));
+    // r and 1/r from one reciprocal square root, each corrected once
+    const double y0 = rsqrt_ulp(r2);
+    const double r0 = mul_(r2, y0);
+    const double r = fma(fma(-r0, r0, r2), 0.5 * y0, r0);
+    k.r = r;
+    k.inv_r = fma(fma(-r, y0, 1.0), y0, y0);
+    const double ct = mul_(z, k.inv_r);
+    const double act = mul_(a, ct);
+    k.inv_sigma = rcp_ulp(fma(act, act, r2));
+    k.inv_ra = rcp_ulp(r2 + a2);
+    k.l[0] = mul_(fma(r, x, mul_(a, y)), k.inv_ra);
+    k.l[1] = mul_(fma(r, y, -mul_(a, x)), k.inv_ra);
+    k.l[2] = ct;
+    k.F = mul_(mul_(2.0 * M, r), k.inv_sigma);
+    const double u = 1.0 + k.F;
+    k.alpha2 = rcp_ulp(u);
+    k.alpha = rsqrt_ulp(u);
+    k.c = mul_(k.F, k.alpha2);
+}
+
+GRHD_HD __forceinline__ void ks_gLL(const KsCell &k, double g[6])
+{
+    const double f[3] = {mul_(k.F, k.l[0]), mul_(k.F, k.l[1]),
+                         mul_(k.F, k.l[2])};
+    g[0] = fma(f[0], k.l[0], 1.0);
+    g[1] = mul_(f[0], k.l[1]);
+    g[2] = mul_(f[0], k.l[2]);
+    g[3] = fma(f[1], k.l[1], 1.0);
+    g[4] = mul_(f[1], k.l[2]);
+    g[5] = fma(f[2], k.l[2], 1.0);
+}
+
+// The face geometry of a cell from them: 60 FP64 operations and five special
+// functions against some 90 and eight of ks_metric's general sequence.
+GRHD_HD __forceinline__ void ks_geo(double M, double a, double x, double y,
+                                    double z, Geo &g)
+{
+    KsCell k;
+    ks_cell(M, a, x, y, z, k);
+    ks_gLL(k, g.gLL);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        g.shift[i] = mul_(k.c, k.l[i]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = i; j < 3; ++j)
+            g.gUU[sym(i, j)] =
+                fma(-g.shift[i], k.l[j], i == j ? 1.0 : 0.0);
+    g.lapse = k.alpha;
+}
+
 // Softened circular-binary potentials at `pos` (add_point_potential,
 // CircularBinaryPN.hpp:252-297).
 template <typename T>
@@ -598,7 +667,14 @@ __device__ __forceinline__ void metric_T(const Background &bg, double x,
                                          double y, double z, GeoT<T> &g,
                                          GeoFullT<T> *f)
 {
-    if constexpr (sizeof(T) == sizeof(double))
+    if constexpr (sizeof(T) == sizeof(double) && !FULL)
+    {
+        if (BGK == 1 || (BGK < 0 && bg.kind == 1))
+            pn_metric<double, false>(bg, x, y, z, g, nullptr);
+        else
+            ks_geo(bg.M, bg.a, x, y, z, g);
+    }
+    else if constexpr (sizeof(T) == sizeof(double))
         background_metric<FULL, BGK>(bg, x, y, z, g, f);
     else
         background_metric_mixed<FULL, BGK>(bg, x, y, z, g, f);
@@ -1104,23 +1180,23 @@ GRHD_HD __forceinline__ T limited_slope(T l, T c, T r, T theta)
 // FP64 members cost the FP32 path a conversion at each use).
 template <typename T> struct FaceOpt
 {
-    T theta, rho_floor, p_floor, vmax2, G, Gm1;
+    T theta; // 0 without reconstruction: every slope is zero
+    T rho_floor, p_floor, vmax2, G, Gm1;
     T Gfac; // G / (G - 1): h = 1 + Gfac p / rho
-    int use_recon;
 };
 
 template <typename T>
 GRHD_HD __forceinline__ FaceOpt<T> make_face_opt(const Options &o)
 {
     FaceOpt<T> f;
-    f.theta = T(o.theta);
+    // (minmod of slopes scaled by a negative theta is zero too)
+    f.theta = o.use_recon && o.theta > 0.0 ? T(o.theta) : T(0);
     f.rho_floor = T(o.rho_floor);
     f.p_floor = T(o.p_floor);
     f.vmax2 = T(o.atmo_vmax2);
     f.G = T(o.G);
     f.Gm1 = T(o.G) - T(1);
     f.Gfac = T(o.G / (o.G - 1.0));
-    f.use_recon = o.use_recon;
     return f;
 }
 
@@ -1143,7 +1219,7 @@ GRHD_HD __forceinline__ double limited_slope_f64(double l, double c, double r,
 #else
     const bool opposite = (dl < 0.0) != (dr < 0.0);
 #endif
-    return opposite || !(theta > 0.0) ? 0.0 : copysign(q, dc);
+    return opposite ? 0.0 : copysign(q, dc);
 }
 
 // One side of an FP64 face: conserved state, physical flux along d and
@@ -1248,10 +1324,16 @@ GRHD_HD __forceinline__ double slope_of(double l, double c, double r,
 {
     return limited_slope_f64(l, c, r, theta);
 }
+// The same in FP32 (limited_slope's value bit for bit while the products of
+// two slopes do not underflow, 1e-45): 14 instructions instead of 21; the
+// mixed face kernel, issue-bound, went from 1.66 to 1.43 ms at 256^3.
 __device__ __forceinline__ float slope_of(float l, float c, float r,
                                           float theta)
 {
-    return limited_slope(l, c, r, theta);
+    const float tl = theta * (c - l), tr = theta * (r - c),
+                dc = 0.5f * (r - l);
+    const float q = fminf(fminf(fabsf(tl), fabsf(tr)), fabsf(dc));
+    return tl * dc > 0.0f && dc * tr > 0.0f ? copysignf(q, dc) : 0.0f;
 }
 
 // The reconstructed values of cell c on its lower and upper faces (MUSCL,
@@ -1265,13 +1347,9 @@ GRHD_HD __forceinline__ void cell_states(const FaceOpt<T> &o,
 #pragma unroll
     for (int q = 0; q < 5; ++q)
     {
-        lower[q] = upper[q] = c.q[q];
-        if (o.use_recon)
-        {
-            const T s = slope_of(l.q[q], c.q[q], r.q[q], o.theta);
-            upper[q] = c.q[q] + T(0.5) * s;
-            lower[q] = c.q[q] - T(0.5) * s;
-        }
+        const T s = slope_of(l.q[q], c.q[q], r.q[q], o.theta);
+        upper[q] = c.q[q] + T(0.5) * s;
+        lower[q] = c.q[q] - T(0.5) * s;
     }
 }
 
@@ -1448,41 +1526,6 @@ GRHD_HD __forceinline__ ConsT<T> static_sources(const PrimT<T> &pr,
 // this, c2p_solve and 32-bit cell indices it holds 128 registers without a
 // spill: 2.77 -> 1.55 ms per launch at 256^3 (bytes alone: 0.72), the RK4
 // step 21.0 -> 15.8 ms.
-struct KsCell
-{
-    double l[3], F, c, alpha, alpha2;
-    double r, inv_r, inv_ra, inv_sigma; // 1/r, 1/(r^2 + a^2), 1/Sigma
-};
-
-GRHD_HD __forceinline__ void ks_cell(double M, double a, double x, double y,
-                                     double z, KsCell &k)
-{
-    const double a2 = mul_(a, a);
-    const double rho2 =
-        fmax(fma(x, x, fma(y, y, mul_(z, z))), 1.0e-12); // (1e-6)^2
-    const double hA = 0.5 * (rho2 - a2);
-    const double az = mul_(a, z);
-    const double r2 = hA + sqrt_(fma(hA, hA, mul_(az, az)));
-    // r and 1/r from one reciprocal square root, each corrected once
-    const double y0 = rsqrt_ulp(r2);
-    const double r0 = mul_(r2, y0);
-    const double r = fma(fma(-r0, r0, r2), 0.5 * y0, r0);
-    k.r = r;
-    k.inv_r = fma(fma(-r, y0, 1.0), y0, y0);
-    const double ct = mul_(z, k.inv_r);
-    const double act = mul_(a, ct);
-    k.inv_sigma = rcp_ulp(fma(act, act, r2));
-    k.inv_ra = rcp_ulp(r2 + a2);
-    k.l[0] = mul_(fma(r, x, mul_(a, y)), k.inv_ra);
-    k.l[1] = mul_(fma(r, y, -mul_(a, x)), k.inv_ra);
-    k.l[2] = ct;
-    k.F = mul_(mul_(2.0 * M, r), k.inv_sigma);
-    const double u = 1.0 + k.F;
-    k.alpha2 = rcp_ulp(u);
-    k.alpha = rsqrt_ulp(u);
-    k.c = mul_(k.F, k.alpha2);
-}
-
 // gamma^ij S_j
 GRHD_HD __forceinline__ void ks_raise(const KsCell &k, const double S[3],
                                       double mU[3])
@@ -1514,18 +1557,6 @@ GRHD_HD __forceinline__ void ks_floors(const Options &o, const KsCell &k,
         pr.v[2] = mul_(pr.v[2], s);
     }
     pr.eps = div_(pr.p, mul_(o.G - 1.0, pr.rho));
-}
-
-GRHD_HD __forceinline__ void ks_gLL(const KsCell &k, double g[6])
-{
-    const double f[3] = {mul_(k.F, k.l[0]), mul_(k.F, k.l[1]),
-                         mul_(k.F, k.l[2])};
-    g[0] = fma(f[0], k.l[0], 1.0);
-    g[1] = mul_(f[0], k.l[1]);
-    g[2] = mul_(f[0], k.l[2]);
-    g[3] = fma(f[1], k.l[1], 1.0);
-    g[4] = mul_(f[1], k.l[2]);
-    g[5] = fma(f[2], k.l[2], 1.0);
 }
 
 GRHD_HD __forceinline__ bool ks_con2prim(const Options &o, const KsCell &k,

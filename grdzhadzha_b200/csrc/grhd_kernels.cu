@@ -709,13 +709,13 @@ __device__ __forceinline__ void block_partial(double v, double *scratch,
 // of planes; every face is evaluated once per tile.  Per plane, two phases
 // between two barriers:
 //   1. the lower x and y face of each thread's cell, from the primitive
-//      tile (2-cell halo, two planes buffered, copied in asynchronously one
-//      plane ahead) and the geometry tile (1-cell halo) in shared memory;
+//      tile (2-cell halo; the planes k to k+2, copied in asynchronously) and
+//      the geometry tile (1-cell halo) in shared memory;
 //      the tile's last x faces fall to warp 0 and its last y faces to warp
 //      1 (the same code once more);
 //   2. the geometry of plane k+1 (own cell in registers and to the tile; the
 //      halo cells fall to warps 2 and 3), the z face above the cell from it,
-//      and the divergence + sources to the RHS.
+//      and the divergence + sources (copied in a plane ahead) to the RHS.
 // The tile needs one geometry buffer: plane k's x and y faces have read it
 // when plane k+1's cells overwrite it, and a z face reads its own column
 // only.  A cell's z slope serves both its z faces: the upper state is
@@ -725,7 +725,9 @@ __device__ __forceinline__ void block_partial(double v, double *scratch,
 // tiles of 15 cells with three barriers, two geometry buffers and the y
 // fluxes stored across the banks, an FP64 RK4 step of the 256^3 torus went
 // from 24.9 to 21.0 ms (mixed 15.9 to 14.9, results unchanged bit for bit),
-// the 64^3 Michel step from 0.68 to 0.55 ms.
+// the 64^3 Michel step from 0.68 to 0.55 ms.  With a third plane buffered (z
+// faces read their column from shared memory instead of waiting for global
+// loads) and the sources prefetched, 2.22 -> 2.00 ms per launch at 256^3.
 // The march starts at plane k0-1 (z face only), so the face below k0 comes
 // from the same code as the block below's upper face, bit for bit: the RHS
 // does not depend on where the z blocks start.
@@ -744,10 +746,11 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
     constexpr int nG = kGW * kGW;
     constexpr int nF = kTC * (kTC + 1); // x or y faces of a tile plane
     constexpr int wX = kTC + 1;         // x faces of a row
-    T *P = reinterpret_cast<T *>(smem_raw); // [2][5][nP]
-    T *G = P + 2 * 5 * nP;                  // [kGeoFields][nG]
+    T *P = reinterpret_cast<T *>(smem_raw); // [3][5][nP], plane mod 3
+    T *G = P + 3 * 5 * nP;                  // [kGeoFields][nG]
     T *Fx = G + kGeoFields * nG;            // [5][nF], row-major rows of wX
     T *Fy = Fx + 5 * nF;                    // [5][nF], kTC + 1 rows of kTC
+    T *Sr = Fy + 5 * nF;                    // [5][256], this plane's sources
     const T idx0 = T(idx0_), idx1 = T(idx1_), idx2 = T(idx2_);
 
     const int a = threadIdx.x, bb = threadIdx.y;
@@ -760,21 +763,22 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
     const bool col_ok = ci <= b.hi[0] && cj <= b.hi[1];
     const int64_t plane = (int64_t)b.gn[0] * b.gn[1];
     const int own_p = (bb + 2) * kPW + a + 2, own_g = (bb + 1) * kGW + a + 1;
-    // this column's primitives at plane k0-2 (clamped into the box)
-    const T *pcol = prim + b.gidx(min(ci, b.hi[0]), min(cj, b.hi[1]), k0 - 2);
-
-    // primitive tiles of planes k0-1 and k0
-    load_p_tile<T, CG, !CG>(P + ((k0 - 1) & 1) * 5 * nP, prim, b, i0, j0,
-                            k0 - 1, tid);
-    load_p_tile<T, CG, !CG>(P + (k0 & 1) * 5 * nP, prim, b, i0, j0, k0, tid);
+    // primitive tiles of planes k0-1, k0 and k0+1; P0, P1, P2 hold the planes
+    // k, k+1, k+2 of the march
+    T *P0 = P, *P1 = P + 5 * nP, *P2 = P + 2 * 5 * nP;
+    load_p_tile<T, CG, !CG>(P0, prim, b, i0, j0, k0 - 1, tid);
+    load_p_tile<T, CG, !CG>(P1, prim, b, i0, j0, k0, tid);
+    load_p_tile<T, CG, !CG>(P2, prim, b, i0, j0, k0 + 1, tid);
     T up[5]; // upper state of the cell at plane k, for the z face above it
     {
+        // this column's primitives from plane k0-2 (clamped into the box)
+        const T *pcol =
+            prim + b.gidx(min(ci, b.hi[0]), min(cj, b.hi[1]), k0 - 2);
         T unused[5];
         cell_states(fo, load_pv_global<T, CG>(pcol, b.pcs, 0),
                     load_pv_global<T, CG>(pcol, b.pcs, plane),
                     load_pv_global<T, CG>(pcol, b.pcs, 2 * plane), unused, up);
     }
-    pcol += 3 * plane; // plane k0+1: plane k+2 of the march's first plane
 
     ConsT<T> Flo = zero_cons<T>();
     double macc = 0.0;
@@ -782,7 +786,6 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
 #pragma unroll 1
     for (int k = k0 - 2; k <= k1; ++k)
     {
-        const T *Pc = P + (k & 1) * 5 * nP;
         const bool zface = k >= k0 - 1; // the z face above plane k
         const bool cells = k >= k0;     // plane k's x/y faces and RHS
         if (cells)
@@ -801,8 +804,8 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
                 geo_sum(G, nG, (fb + 1) * kGW + fa, (fb + 1) * kGW + fa + 1, 0,
                         gf);
                 const ConsT<T> f = face_flux(
-                    fo, load_pv_smem(Pc, row), load_pv_smem(Pc, row + 1),
-                    load_pv_smem(Pc, row + 2), load_pv_smem(Pc, row + 3), gf,
+                    fo, load_pv_smem(P0, row), load_pv_smem(P0, row + 1),
+                    load_pv_smem(P0, row + 2), load_pv_smem(P0, row + 3), gf,
                     0);
                 const int fi = fb * wX + fa;
                 if (MDOT && fa < kTC && i0 + fa <= b.hi[0])
@@ -828,9 +831,9 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
                 geo_sum(G, nG, fb * kGW + fa + 1, (fb + 1) * kGW + fa + 1, 1,
                         gf);
                 const ConsT<T> f = face_flux(
-                    fo, load_pv_smem(Pc, col), load_pv_smem(Pc, col + kPW),
-                    load_pv_smem(Pc, col + 2 * kPW),
-                    load_pv_smem(Pc, col + 3 * kPW), gf, 1);
+                    fo, load_pv_smem(P0, col), load_pv_smem(P0, col + kPW),
+                    load_pv_smem(P0, col + 2 * kPW),
+                    load_pv_smem(P0, col + 3 * kPW), gf, 1);
                 const int fi = fb * kTC + fa;
                 if (MDOT && fb < kTC && j0 + fb <= b.hi[1])
                     macc +=
@@ -842,24 +845,19 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
                 Fy[4 * nF + fi] = f.tau;
             }
         }
-        // this column's primitives at planes k and k+2 of the face above
-        PVT<T> w1, w3;
+        // this column's primitives at plane k, whose tile gives way to
+        // plane k+3's
+        PVT<T> w1;
         if (zface)
-        {
-            w1 = load_pv_smem(Pc, own_p);
-            w3 = load_pv_global<T, CG>(pcol, b.pcs, 0);
-            pcol += plane;
-        }
-        // plane k+1's tile, issued one plane ago (the first two before the
-        // march), has landed
+            w1 = load_pv_smem(P0, own_p);
+        // plane k+2's tile and plane k's sources, issued one plane ago, have
+        // landed
         if (!CG)
             cp_async_wait_all();
         __syncthreads();
-        // plane k's tile has been read: fetch plane k+2's into its place
-        // (of plane k1+1 the z faces read their own columns)
+        // of the planes above k1 the z faces read their own columns only
         if (zface && k < k1)
-            load_p_tile<T, CG, !CG>(P + (k & 1) * 5 * nP, prim, b, i0, j0,
-                                    k + 2, tid);
+            load_p_tile<T, CG, !CG>(P0, prim, b, i0, j0, k + 3, tid);
         // geometry of plane k+1: the halo cells (where the next plane has x
         // and y faces), then the own cell, left in registers
         GeoT<T> gn;
@@ -889,9 +887,9 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
         {
             GeoT<T> gf;
             geo_sum_z(G, nG, own_g, gn, gf);
-            const PVT<T> w2 = load_pv_smem(P + ((k + 1) & 1) * 5 * nP, own_p);
             T low[5], next[5];
-            cell_states(fo, w1, w2, w3, low, next);
+            cell_states(fo, w1, load_pv_smem(P1, own_p),
+                        load_pv_smem(P2, own_p), low, next);
             Fhi = state_flux(fo, up, low, gf, 2);
 #pragma unroll
             for (int c = 0; c < 5; ++c)
@@ -917,7 +915,9 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
                 const T ry =
                     -idx1 * (Fy[c * nF + fy + kTC] - Fy[c * nF + fy]);
                 const T rz = -idx2 * (fh[c] - fl[c]);
-                out[c] = ((rx + ry) + rz) + rdro<CG>(&src[c * b.rcs + ri]);
+                out[c] = ((rx + ry) + rz) +
+                         (CG ? rdro<CG>(&src[c * b.rcs + ri])
+                             : Sr[c * (kTB * kTB) + tid]);
             }
             if (excised(o, ci, cj, k))
             {
@@ -930,6 +930,22 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
                 rhs[c * b.rcs + ri] = out[c];
         }
         Flo = Fhi;
+        // the next plane's sources of this cell
+        if (!CG && zface && k < k1 && col_ok)
+        {
+            const int64_t ri = b.iidx(ci, cj, k + 1);
+#pragma unroll
+            for (int c = 0; c < 5; ++c)
+                cp_async_elem(&Sr[c * (kTB * kTB) + tid],
+                              &src[c * b.rcs + ri]);
+        }
+        if (zface)
+        {
+            T *const p = P0;
+            P0 = P1;
+            P1 = P2;
+            P2 = p;
+        }
         __syncthreads();
     }
     if (MDOT)
@@ -975,14 +991,16 @@ __global__ void k_mdot_sum(const double *__restrict__ part, int64_t n,
 
 // recover_primitives_and_apply_atmosphere_from_fixed_background for one
 // cell (FixedBGFArrayBoxFiniteVolume.hpp:60-110); c is the updated
-// conserved state.  Writes prims (and reset conserved) to `out`.
+// conserved state.  Writes prims (and reset conserved) to `out`.  T picks the
+// path's root solve (the metric is FP64 in both).
+template <typename T>
 __device__ __forceinline__ void recover_cell(const Options &o, const Geo &g,
                                              Cons c, double *out, int64_t cs,
                                              int64_t idx,
                                              unsigned long long cnt[4])
 {
     Prim pr;
-    const bool ok = con2prim(o, c, g.gUU, pr, nullptr, nullptr);
+    const bool ok = cold_con2prim<T>(o, c, g.gUU, pr);
     bool reset = !ok;
     cnt[0] += 1;
     if (ok)
@@ -1032,6 +1050,7 @@ __device__ __forceinline__ void flush_counts(DevStatus *st,
 // update_conserved: dst = src + dt * rhs on the interior
 // (add_scaled_conserved_rhs, FArrayBoxFiniteVolume.hpp:927-940), then the
 // post-update recovery when `recover` is set.
+template <typename T>
 __global__ void __launch_bounds__(256)
     k_update(double *dst, int64_t dcs, const double *srcs, int64_t scs,
              const double *__restrict__ rhs, BoxDev b, Background bg,
@@ -1068,7 +1087,7 @@ __global__ void __launch_bounds__(256)
                     cell_xyz(o, i, j, k, x, y, z);
                     Geo geo;
                     background_metric<false>(bg, x, y, z, geo, nullptr);
-                    recover_cell(o, geo, c, dst, dcs, g, cnt);
+                    recover_cell<T>(o, geo, c, dst, dcs, g, cnt);
                 }
                 else
                 {
@@ -1083,6 +1102,7 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+template <typename T>
 __global__ void __launch_bounds__(256)
     k_recover(double *__restrict__ state, BoxDev b, Background bg, Options o,
               DevStatus *st)
@@ -1104,8 +1124,8 @@ __global__ void __launch_bounds__(256)
                 cell_xyz(o, i, j, k, x, y, z);
                 Geo geo;
                 background_metric<false>(bg, x, y, z, geo, nullptr);
-                recover_cell(o, geo, load_cons(state, b.cs, g), state, b.cs,
-                             g, cnt);
+                recover_cell<T>(o, geo, load_cons(state, b.cs, g), state, b.cs,
+                                g, cnt);
             }
         }
         flush_counts(st, cnt);
@@ -2032,8 +2052,8 @@ int grid_for(int64_t n, int threads)
 template <typename T> size_t faces_smem()
 {
     return sizeof(T) *
-           (2 * 5 * kPW * kPW + kGeoFields * kGW * kGW +
-            2 * 5 * kTC * (kTC + 1));
+           (3 * 5 * kPW * kPW + kGeoFields * kGW * kGW +
+            2 * 5 * kTC * (kTC + 1) + 5 * kTB * kTB);
 }
 
 // ---------------------------------------------- CCZ4-stored geometry
@@ -2352,7 +2372,8 @@ __global__ void __launch_bounds__(256)
             const int64_t g = b.gidx(i, j, k);
             Geo geo;
             ccz4_geo(s, b.cs, g, geo, nullptr);
-            recover_cell(o, geo, load_cons(q, b.cs, g), q, b.cs, g, cnt);
+            recover_cell<double>(o, geo, load_cons(q, b.cs, g), q, b.cs, g,
+                                 cnt);
         }
         flush_counts(st, cnt);
         cnt[0] = cnt[1] = cnt[2] = cnt[3] = 0;
@@ -2704,16 +2725,23 @@ void launch_mdot_sum(const double *part, int64_t n, double weight,
 void launch_update(double *dst, int64_t dcs, const double *src_state,
                    int64_t scs, const double *rhs, const BoxDev &b,
                    const Background &bg, const Options &o, double dt,
-                   int recover, DevStatus *st, cudaStream_t s)
+                   int recover, DevStatus *st, bool mixed, cudaStream_t s)
 {
-    k_update<<<grid_for(b.ivol(), 256), 256, 0, s>>>(
-        dst, dcs, src_state, scs, rhs, b, bg, o, dt, recover, st);
+    auto go = [&](auto kern) {
+        kern<<<grid_for(b.ivol(), 256), 256, 0, s>>>(
+            dst, dcs, src_state, scs, rhs, b, bg, o, dt, recover, st);
+    };
+    mixed ? go(k_update<float>) : go(k_update<double>);
 }
 
 void launch_recover(double *state, const BoxDev &b, const Background &bg,
-                    const Options &o, DevStatus *st, cudaStream_t s)
+                    const Options &o, DevStatus *st, bool mixed,
+                    cudaStream_t s)
 {
-    k_recover<<<grid_for(b.ivol(), 256), 256, 0, s>>>(state, b, bg, o, st);
+    auto go = [&](auto kern) {
+        kern<<<grid_for(b.ivol(), 256), 256, 0, s>>>(state, b, bg, o, st);
+    };
+    mixed ? go(k_recover<float>) : go(k_recover<double>);
 }
 
 // Blocks of a stage launch: two cells a thread where that leaves four waves
