@@ -170,6 +170,11 @@ template <typename T>
 void launch_cells(const double *state, T *prim, T *src, const BoxDev &b,
                   const Background &bg, const Options &o, DevStatus *st,
                   cudaStream_t s);
+// launch_fill_ghosts and launch_cells in one launch (FP64), for boxes small
+// enough that this pays; false (nothing launched) for others.
+bool launch_prepare(double *state, double *prim, double *src, const BoxDev &b,
+                    const Background &bg, const Options &o, DevStatus *st,
+                    cudaStream_t s);
 // Face fluxes + divergence + sources -> rhs.  mdot_part (one double per
 // block) receives the block sums of the accretion-rate faces when
 // o.accretion_radius > 0.
