@@ -2063,11 +2063,10 @@ int grhd_kitp_advance_ssprk2(grhd_ctx *ctx, double *state, int64_t state_cs,
                         0.5 * dt);
     if (visc)
         launch_kitp_viscous_rhs(k, b.ivol(), ctx->stage, sb, ctx->opt, k1, s);
-    launch_kitp_combine(state, b, ctx->stage, sb.cs, k, b.ivol(), dt, s);
-    if (cfg->sink_rate != 0.0 && cfg->sink_size > 0.0)
-        launch_kitp_sink_decay(state, b, ctx->opt, kh, dt, s);
-    launch_recover(state, b, bg1, ctx->opt, ctx->status, false, s);
-    ctx->launches += 4 + (visc ? 2 : 0);
+    launch_kitp_finish(state, b, ctx->stage, sb.cs, k, b.ivol(), bg1, ctx->opt,
+                       kh, cfg->sink_rate != 0.0 && cfg->sink_size > 0.0, dt,
+                       ctx->status, s);
+    ctx->launches += 2 + (visc ? 2 : 0);
     st = finish_status(ctx, b, state, bg0, s);
     read_diag(ctx, diag);
     return st;

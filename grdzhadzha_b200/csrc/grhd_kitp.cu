@@ -17,28 +17,6 @@ __device__ __forceinline__ void cell_of_interior(const BoxDev &b, int64_t t,
     k = b.lo[2] + (int)(r / b.in[1]);
 }
 
-// sink_kernel (:557-565) summed over both bodies (:584-597)
-__device__ double sink_rate(const KitpDev &k, double x, double y, double z)
-{
-    const double pos[3] = {x, y, z};
-    double rate = 0.0;
-    for (int body = 0; body < 2; ++body)
-    {
-        double r2 = 0.0;
-        for (int d = 0; d < 3; ++d)
-        {
-            const double dd = pos[d] - k.body[body][d];
-            r2 += dd * dd;
-        }
-        const double radius = k.sink_size * k.mass[body];
-        double kern = 0.0;
-        if (radius > 0.0 && k.sink_rate != 0.0)
-            kern = exp(-pow(r2 / (radius * radius), 0.5 * k.sink_shape));
-        rate += k.sink_rate * kern;
-    }
-    return rate;
-}
-
 __device__ __forceinline__ int clampi(int v, int lo, int hi)
 {
     return v < lo ? lo : (v > hi ? hi : v);
@@ -59,19 +37,21 @@ __device__ double dynamic_viscosity(const KitpDev &k, const Options &o,
             const double dd = pos[d] - k.body[body][d];
             r2 += dd * dd;
         }
-        omega2 += k.mass[body] * pow(r2, -1.5);
+        const double y = rsqrt_(r2);
+        omega2 += k.mass[body] * (y * y * y);
     }
-    const double cs2 = o.G * p / fmax(rho, k.rho_floor_cfg);
-    return rho * k.alpha * cs2 / sqrt(fmax(omega2, 1.0e-300));
+    const double cs2 = div_(o.G * p, fmax(rho, k.rho_floor_cfg));
+    return rho * k.alpha * cs2 * rsqrt_(fmax(omega2, 1.0e-300));
 }
 
-// viscous_flux_for_cell (:700-770) of cell (i,j,l) in direction dir:
-// f[0], f[1] the S_x, S_y fluxes, f[2] the tau flux.
-__device__ void viscous_flux(const double *__restrict__ s, const BoxDev &b,
-                             const Options &o, const KitpDev &k, int i, int j,
-                             int l, int dir, double f[3])
+// The viscous fluxes of cell (i,j,l) in both directions
+// (viscous_flux_for_cell, :700-770): f = (F_x[S_x], F_x[S_y] = F_y[S_x],
+// F_y[S_y], F_x[tau], F_y[tau]).
+__device__ void viscous_fluxes(const double *__restrict__ s, const BoxDev &b,
+                               const Options &o, const KitpDev &k, int i,
+                               int j, int l, double f[5])
 {
-    f[0] = f[1] = f[2] = 0.0;
+    f[0] = f[1] = f[2] = f[3] = f[4] = 0.0;
     const int64_t g = b.gidx(i, j, l);
     const double rho = __ldg(&s[kRho * b.cs + g]);
     if (rho <= 10.0 * k.atmo_rho_floor)
@@ -83,68 +63,98 @@ __device__ void viscous_flux(const double *__restrict__ s, const BoxDev &b,
         dynamic_viscosity(k, o, rho, __ldg(&s[kPress * b.cs + g]), pos);
     if (mu == 0.0)
         return;
-    const int iv[3] = {i, j, l};
+    const int iv[2] = {i, j};
+    const int64_t step[2] = {1, b.gn[0]};
     double gradv[2][2];
     for (int c = 0; c < 2; ++c)
     {
-        int m[3] = {i, j, l}, q[3] = {i, j, l};
-        m[c] = clampi(iv[c] - 1, b.dlo[c], b.dhi[c]);
-        q[c] = clampi(iv[c] + 1, b.dlo[c], b.dhi[c]);
-        const int span = q[c] - m[c];
+        const int m = clampi(iv[c] - 1, b.dlo[c], b.dhi[c]) - iv[c];
+        const int q = clampi(iv[c] + 1, b.dlo[c], b.dhi[c]) - iv[c];
+        const int span = q - m;
         const double den = (span > 1 ? span : 1) * o.dx;
-        const int64_t gm = b.gidx(m[0], m[1], m[2]);
-        const int64_t gq = b.gidx(q[0], q[1], q[2]);
         for (int v = 0; v < 2; ++v)
-            gradv[v][c] = (__ldg(&s[(kV1 + v) * b.cs + gq]) -
-                           __ldg(&s[(kV1 + v) * b.cs + gm])) /
-                          den;
+            gradv[v][c] = div_(__ldg(&s[(kV1 + v) * b.cs + g + q * step[c]]) -
+                                   __ldg(&s[(kV1 + v) * b.cs + g +
+                                            m * step[c]]),
+                               den);
     }
     const double divergence = gradv[0][0] + gradv[1][1];
-    double tau[2][2];
-    for (int a = 0; a < 2; ++a)
-        for (int c = 0; c < 2; ++c)
-            tau[a][c] = mu * (gradv[a][c] + gradv[c][a] +
-                              (k.beta - 2.0 / 3.0) * (double)(a == c) *
-                                  divergence);
+    const double bulk = (k.beta - 2.0 / 3.0) * divergence;
+    const double xx = mu * (gradv[0][0] + gradv[0][0] + bulk);
+    const double xy = mu * (gradv[0][1] + gradv[1][0]);
+    const double yy = mu * (gradv[1][1] + gradv[1][1] + bulk);
     const double vx = __ldg(&s[kV1 * b.cs + g]);
     const double vy = __ldg(&s[(kV1 + 1) * b.cs + g]);
-    f[0] = -tau[dir][0];
-    f[1] = -tau[dir][1];
-    f[2] = -tau[dir][0] * vx - tau[dir][1] * vy;
+    f[0] = -xx;
+    f[1] = -xy;
+    f[2] = -yy;
+    f[3] = -xx * vx - xy * vy;
+    f[4] = -xy * vx - yy * vy;
 }
 
-__global__ void __launch_bounds__(256)
+// A block owns 32 x 8 cells of a plane and evaluates the fluxes of its cells
+// and their x and y neighbours once, into shared memory (1.3 evaluations a
+// cell; one thread per cell evaluating its four neighbours took 141 us at
+// 128 x 128 x 48, three quarters of it in pow; now 30).
+constexpr int kVX = 32, kVY = 8;
+
+__global__ void __launch_bounds__(kVX *kVY)
     k_kitp_viscous(double *__restrict__ rhs, int64_t rcs,
                    const double *__restrict__ s, BoxDev b, Options o,
                    KitpDev k)
 {
-    const int64_t n = b.ivol();
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
-         t += (int64_t)gridDim.x * blockDim.x)
+    constexpr int W = kVX + 2, n = W * (kVY + 2);
+    __shared__ double F[5][n];
+    const int i0 = b.lo[0] + blockIdx.x * kVX;
+    const int j0 = b.lo[1] + blockIdx.y * kVY;
+    const int tid = threadIdx.y * kVX + threadIdx.x;
+    const double w = 1.0 / (2.0 * o.dx);
+    for (int l = b.lo[2] + blockIdx.z; l <= b.hi[2]; l += gridDim.z)
     {
-        int i, j, l;
-        cell_of_interior(b, t, i, j, l);
-        const int iv[3] = {i, j, l};
-        for (int d = 0; d < 2; ++d)
+        for (int q = tid; q < n; q += kVX * kVY)
         {
-            int lo[3] = {i, j, l}, hi[3] = {i, j, l};
-            lo[d] = clampi(iv[d] - 1, b.dlo[d], b.dhi[d]);
-            hi[d] = clampi(iv[d] + 1, b.dlo[d], b.dhi[d]);
-            double fl[3], fh[3];
-            viscous_flux(s, b, o, k, lo[0], lo[1], lo[2], d, fl);
-            viscous_flux(s, b, o, k, hi[0], hi[1], hi[2], d, fh);
-            rhs[4 * rcs + t] -= (fh[2] - fl[2]) / (2.0 * o.dx);
-            rhs[1 * rcs + t] -= (fh[0] - fl[0]) / (2.0 * o.dx);
-            rhs[2 * rcs + t] -= (fh[1] - fl[1]) / (2.0 * o.dx);
+            const int u = q % W, v = q / W;
+            const int i = i0 - 1 + u, j = j0 - 1 + v;
+            const bool corner =
+                (u == 0 || u == W - 1) && (v == 0 || v == kVY + 1);
+            // cells beyond the domain stand for their clamped neighbours,
+            // cells beyond the box's neighbours are not read
+            if (corner || i < b.dlo[0] || i > b.dhi[0] || j < b.dlo[1] ||
+                j > b.dhi[1] || i > b.hi[0] + 1 || j > b.hi[1] + 1)
+                continue;
+            double f[5];
+            viscous_fluxes(s, b, o, k, i, j, l, f);
+#pragma unroll
+            for (int c = 0; c < 5; ++c)
+                F[c][q] = f[c];
         }
+        __syncthreads();
+        const int i = i0 + threadIdx.x, j = j0 + threadIdx.y;
+        if (i <= b.hi[0] && j <= b.hi[1])
+        {
+            const int at = (threadIdx.y + 1) * W + threadIdx.x + 1;
+            const int xl = at + clampi(i - 1, b.dlo[0], b.dhi[0]) - i;
+            const int xh = at + clampi(i + 1, b.dlo[0], b.dhi[0]) - i;
+            const int yl = at + W * (clampi(j - 1, b.dlo[1], b.dhi[1]) - j);
+            const int yh = at + W * (clampi(j + 1, b.dlo[1], b.dhi[1]) - j);
+            const int64_t t = b.iidx(i, j, l);
+            rhs[1 * rcs + t] = rhs[1 * rcs + t] - (F[0][xh] - F[0][xl]) * w -
+                               (F[1][yh] - F[1][yl]) * w;
+            rhs[2 * rcs + t] = rhs[2 * rcs + t] - (F[1][xh] - F[1][xl]) * w -
+                               (F[2][yh] - F[2][yl]) * w;
+            rhs[4 * rcs + t] = rhs[4 * rcs + t] - (F[3][xh] - F[3][xl]) * w -
+                               (F[4][yh] - F[4][yl]) * w;
+        }
+        __syncthreads();
     }
 }
 
 __global__ void __launch_bounds__(256)
     k_kitp_sink_rhs(double *__restrict__ rhs, int64_t rcs,
                     const double *__restrict__ s, BoxDev b, Options o,
-                    KitpDev k)
+                    KitpDev k, double r2max0, double r2max1)
 {
+    const double r2max[2] = {r2max0, r2max1};
     const int64_t n = b.ivol();
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
          t += (int64_t)gridDim.x * blockDim.x)
@@ -156,7 +166,7 @@ __global__ void __launch_bounds__(256)
             continue;
         double x, y, z;
         cell_xyz(o, i, j, l, x, y, z);
-        const double rate = sink_rate(k, x, y, z);
+        const double rate = kitp_sink(k, r2max, x, y, z);
         if (rate == 0.0)
             continue;
         rhs[0 * rcs + t] -= rate * s[kD * b.cs + g];
@@ -168,8 +178,9 @@ __global__ void __launch_bounds__(256)
 
 __global__ void __launch_bounds__(256)
     k_kitp_sink_decay(double *__restrict__ s, BoxDev b, Options o, KitpDev k,
-                      double dt)
+                      double dt, double r2max0, double r2max1)
 {
+    const double r2max[2] = {r2max0, r2max1};
     const int64_t n = b.ivol();
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
          t += (int64_t)gridDim.x * blockDim.x)
@@ -181,7 +192,7 @@ __global__ void __launch_bounds__(256)
             continue;
         double x, y, z;
         cell_xyz(o, i, j, l, x, y, z);
-        const double rate = sink_rate(k, x, y, z);
+        const double rate = kitp_sink(k, r2max, x, y, z);
         if (rate == 0.0)
             continue;
         const double decay = exp(-rate * dt);
@@ -283,25 +294,6 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-__global__ void __launch_bounds__(256)
-    k_kitp_combine(double *__restrict__ s, BoxDev b,
-                   const double *__restrict__ u1, int64_t ucs,
-                   const double *__restrict__ k, int64_t rcs, double dt)
-{
-    const int64_t n = b.ivol();
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
-         t += (int64_t)gridDim.x * blockDim.x)
-    {
-        int i, j, l;
-        cell_of_interior(b, t, i, j, l);
-        const int64_t g = b.gidx(i, j, l);
-        // RHS components D, S1..3, tau are the state's first five
-        for (int c = 0; c < 5; ++c)
-            s[c * b.cs + g] =
-                0.5 * (s[c * b.cs + g] + u1[c * ucs + g] + dt * k[c * rcs + t]);
-    }
-}
-
 int blocks_for(int64_t n)
 {
     int64_t g = (n + 255) / 256;
@@ -316,23 +308,28 @@ void launch_kitp_viscous_rhs(double *rhs, int64_t rcs, const double *state,
                              const BoxDev &b, const Options &o,
                              const KitpDev &k, cudaStream_t s)
 {
-    k_kitp_viscous<<<blocks_for(b.ivol()), 256, 0, s>>>(rhs, rcs, state, b, o,
-                                                        k);
+    const dim3 grid((b.in[0] + kVX - 1) / kVX, (b.in[1] + kVY - 1) / kVY,
+                    b.in[2] < 65535 ? b.in[2] : 65535);
+    k_kitp_viscous<<<grid, dim3(kVX, kVY), 0, s>>>(rhs, rcs, state, b, o, k);
 }
 
 void launch_kitp_sink_rhs(double *rhs, int64_t rcs, const double *state,
                           const BoxDev &b, const Options &o, const KitpDev &k,
                           cudaStream_t s)
 {
-    k_kitp_sink_rhs<<<blocks_for(b.ivol()), 256, 0, s>>>(rhs, rcs, state, b,
-                                                         o, k);
+    double r2max[2];
+    kitp_sink_reach(k, r2max);
+    k_kitp_sink_rhs<<<blocks_for(b.ivol()), 256, 0, s>>>(
+        rhs, rcs, state, b, o, k, r2max[0], r2max[1]);
 }
 
 void launch_kitp_sink_decay(double *state, const BoxDev &b, const Options &o,
                             const KitpDev &k, double dt, cudaStream_t s)
 {
-    k_kitp_sink_decay<<<blocks_for(b.ivol()), 256, 0, s>>>(state, b, o, k,
-                                                           dt);
+    double r2max[2];
+    kitp_sink_reach(k, r2max);
+    k_kitp_sink_decay<<<blocks_for(b.ivol()), 256, 0, s>>>(
+        state, b, o, k, dt, r2max[0], r2max[1]);
 }
 
 void launch_kitp_disk_fill(double *state, const BoxDev &b,
@@ -340,14 +337,6 @@ void launch_kitp_disk_fill(double *state, const BoxDev &b,
                            const KitpDiskDev &k, cudaStream_t s)
 {
     k_kitp_disk_fill<<<blocks_for(b.gvol()), 256, 0, s>>>(state, b, bg, o, k);
-}
-
-void launch_kitp_combine(double *state, const BoxDev &b, const double *u1,
-                         int64_t u1_cs, const double *k, int64_t rcs,
-                         double dt, cudaStream_t s)
-{
-    k_kitp_combine<<<blocks_for(b.ivol()), 256, 0, s>>>(state, b, u1, u1_cs, k,
-                                                        rcs, dt);
 }
 
 } // namespace grhd
