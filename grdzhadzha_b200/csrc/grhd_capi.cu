@@ -37,9 +37,9 @@ struct grhd_ctx
     size_t stage_cap = 0;
     double *diag_part = nullptr;  // diagnostics: per-block partial results
     size_t diag_cap = 0;
-    double *ccz4_geo = nullptr;   // CCZ4 operator: geometry cache (16 comps)
+    double *ccz4_geo = nullptr;   // CCZ4 operator: geometry cache
     size_t ccz4_geo_cap = 0;
-    double *ccz4_stage = nullptr; // CCZ4 operator: SSPRK2 stage (36 comps)
+    double *ccz4_stage = nullptr; // CCZ4 operator: SSPRK2 stage (GRHD)
     size_t ccz4_stage_cap = 0;
     double *host_state = nullptr; // device copy of a host-held state
     size_t host_state_cap = 0;
@@ -971,25 +971,34 @@ int ccz4_checks(grhd_ctx *ctx, const double *state, int64_t state_cs,
     if ((st = check_strides(ctx, b, state_cs, rhs_cs)) ||
         (st = ensure_scratch(ctx, b, false)) ||
         (st = grow(ctx, &ctx->ccz4_geo, &ctx->ccz4_geo_cap,
-                   16 * (size_t)b.gvol())) ||
+                   kCcz4GeoFields * (size_t)b.gvol())) ||
         (st = reset_status(ctx, s)))
         return st;
     return GRHD_OK;
 }
 
-// compute_leveldata_flux_rhs_from_ccz4_geometry (:1047-1090) on one box:
-// the fills, the ghosted-box recovery into the caches, then one kernel for
-// the three directional flux differences and the sources.
-void enqueue_ccz4_rhs(grhd_ctx *ctx, double *rhs, int64_t rhs_cs,
-                      double *state, const BoxDev &b,
+double *grhd_part(double *state, int64_t cs)
+{
+    return state + kCcz4GrhdOffset * cs;
+}
+
+// compute_leveldata_flux_rhs_from_ccz4_geometry (:1047-1090) on one box: the
+// fills, the ghosted-box recovery into the caches, the sources and the
+// directional flux differences.  `metric` holds the CCZ4 components, q the
+// GRHD ones; with qp = null the metric is new to the caches, else q is a
+// stage state on the same metric whose ghosts take their primitives from qp
+// (stride pcs).  rhs has stride b.rcs = the interior volume.
+void enqueue_ccz4_rhs(grhd_ctx *ctx, double *rhs, double *metric,
+                      const BoxDev &b, double *q, int64_t qcs,
+                      const double *qp, int64_t pcs,
                       const double inverse_dx[3], cudaStream_t s)
 {
-    launch_ccz4_fill(state, b, true, s);
-    launch_ccz4_cells(state, b, ctx->opt, ctx->prim, ctx->ccz4_geo,
-                      ctx->status, s);
-    launch_ccz4_rhs(state, b, ctx->opt, ctx->prim, ctx->ccz4_geo, rhs, rhs_cs,
-                    inverse_dx, ctx->status, s);
-    ctx->launches += 3;
+    launch_ccz4_fill(qp ? nullptr : metric, b.cs, q, qcs, qp, pcs, b, s);
+    launch_ccz4_cells(metric, b.cs, q, qcs, b, ctx->opt, ctx->prim,
+                      ctx->ccz4_geo, !qp, ctx->status, s);
+    launch_ccz4_rhs(metric, b.cs, q, qcs, b, ctx->opt, ctx->prim,
+                    ctx->ccz4_geo, ctx->src, rhs, inverse_dx, s);
+    ctx->launches += 4;
 }
 
 // ---- the host-buffer RK4 step as a wavefront over z chunks
@@ -1202,7 +1211,16 @@ int grhd_ccz4_compute_rhs(grhd_ctx *ctx, double *rhs, int64_t rhs_cs,
     int st = ccz4_checks(ctx, state, state_cs, box, rhs_cs, b, s);
     if (st)
         return st;
-    enqueue_ccz4_rhs(ctx, rhs, rhs_cs, state, b, inverse_dx, s);
+    // the kernels write with the interior-volume stride
+    double *out = rhs_cs == b.ivol() ? rhs : ctx->kbuf;
+    enqueue_ccz4_rhs(ctx, out, state, b, grhd_part(state, b.cs), b.cs, nullptr,
+                     0, inverse_dx, s);
+    if (out != rhs)
+        for (int c = 0; c < 5; ++c)
+            GRHD_CUDA(ctx, cudaMemcpyAsync(rhs + c * rhs_cs,
+                                           out + c * b.ivol(),
+                                           b.ivol() * sizeof(double),
+                                           cudaMemcpyDeviceToDevice, s));
     return ccz4_finish(ctx, b, state, s);
 }
 
@@ -1239,7 +1257,7 @@ int grhd_ccz4_update_conserved(grhd_ctx *ctx, double *state,
     int st = ccz4_checks(ctx, state, state_cs, box, rhs_cs, b, s);
     if (st)
         return st;
-    launch_ccz4_update(state, nullptr, 0, rhs, rhs_cs, b, dt, 0, s);
+    launch_ccz4_update(state, rhs, rhs_cs, b, dt, s);
     ++ctx->launches;
     if (recover)
     {
@@ -1293,26 +1311,22 @@ int grhd_ccz4_advance_ssprk2(grhd_ctx *ctx, double *state, int64_t state_cs,
         return st;
     const int64_t gv = b.gvol();
     if ((st = grow(ctx, &ctx->ccz4_stage, &ctx->ccz4_stage_cap,
-                   (size_t)GRHD_CCZ4_NUM_VARS * gv)))
+                   (size_t)kStateComps * gv)))
         return st;
-    BoxDev sb = b;
-    sb.cs = gv;
-    double *stage = ctx->ccz4_stage;
-    double *k0 = ctx->kbuf, *k1 = ctx->src; // rhs_initial, rhs_stage
     // advance_ssprk2 (:1323-1348): stage = state; rhs_initial = L(state);
     // stage += dt rhs_initial, recovered; rhs_stage = L(stage);
-    // state = (state + stage + dt rhs_stage) / 2, recovered
-    GRHD_CUDA(ctx, cudaMemcpy2DAsync(stage, gv * sizeof(double), state,
-                                     state_cs * sizeof(double),
-                                     gv * sizeof(double), GRHD_CCZ4_NUM_VARS,
-                                     cudaMemcpyDeviceToDevice, s));
-    enqueue_ccz4_rhs(ctx, k0, b.ivol(), state, b, inverse_dx, s);
-    launch_ccz4_update(stage, nullptr, 0, k0, b.ivol(), sb, dt, 0, s);
-    launch_ccz4_recover(stage, sb, ctx->opt, ctx->status, s);
-    enqueue_ccz4_rhs(ctx, k1, b.ivol(), stage, sb, inverse_dx, s);
-    launch_ccz4_update(state, stage, gv, k1, b.ivol(), b, dt, 1, s);
-    launch_ccz4_recover(state, b, ctx->opt, ctx->status, s);
-    ctx->launches += 4;
+    // state = (state + stage + dt rhs_stage) / 2, recovered.  The stage
+    // state is its GRHD components on the state's metric.
+    double *q = grhd_part(state, b.cs), *stage = ctx->ccz4_stage;
+    double *k = ctx->kbuf;
+    enqueue_ccz4_rhs(ctx, k, state, b, q, b.cs, nullptr, 0, inverse_dx, s);
+    launch_ccz4_advance(stage, gv, q, b.cs, nullptr, 0, k, b.ivol(), b,
+                        ctx->opt, ctx->ccz4_geo, nullptr, 0, dt, ctx->status,
+                        s);
+    enqueue_ccz4_rhs(ctx, k, state, b, stage, gv, q, b.cs, inverse_dx, s);
+    launch_ccz4_advance(q, b.cs, q, b.cs, stage, gv, k, b.ivol(), b, ctx->opt,
+                        ctx->ccz4_geo, nullptr, 0, dt, ctx->status, s);
+    ctx->launches += 2;
     st = ccz4_finish(ctx, b, state, s);
     read_diag(ctx, diag);
     return st;
@@ -1349,22 +1363,26 @@ int grhd_ccz4_ssprk2_stage(grhd_ctx *ctx, int stage, double *state,
                                          gv * sizeof(double),
                                          GRHD_CCZ4_NUM_VARS,
                                          cudaMemcpyDeviceToDevice, s));
-        enqueue_ccz4_rhs(ctx, ctx->kbuf, b.ivol(), state, b, inverse_dx, s);
-        launch_ccz4_update(stage_state, nullptr, 0, ctx->kbuf, b.ivol(), sb,
-                           dt, 0, s);
-        launch_ccz4_recover(stage_state, sb, ctx->opt, ctx->status, s);
+        double *q = grhd_part(state, b.cs);
+        enqueue_ccz4_rhs(ctx, ctx->kbuf, state, b, q, b.cs, nullptr, 0,
+                         inverse_dx, s);
+        launch_ccz4_advance(grhd_part(stage_state, stage_cs), stage_cs, q,
+                            b.cs, nullptr, 0, ctx->kbuf, b.ivol(), b, ctx->opt,
+                            ctx->ccz4_geo, nullptr, 0, dt, ctx->status, s);
     }
     else
     {
         // rhs_stage = L(stage); state = (state + stage + dt rhs_stage) / 2,
-        // recovered
-        enqueue_ccz4_rhs(ctx, ctx->kbuf, b.ivol(), stage_state, sb,
-                         inverse_dx, s);
-        launch_ccz4_update(state, stage_state, stage_cs, ctx->kbuf, b.ivol(),
-                           b, dt, 1, s);
-        launch_ccz4_recover(state, b, ctx->opt, ctx->status, s);
+        // recovered on the state's metric
+        double *q = grhd_part(state, b.cs);
+        double *qs = grhd_part(stage_state, stage_cs);
+        enqueue_ccz4_rhs(ctx, ctx->kbuf, stage_state, sb, qs, stage_cs,
+                         nullptr, 0, inverse_dx, s);
+        launch_ccz4_advance(q, b.cs, q, b.cs, qs, stage_cs, ctx->kbuf,
+                            b.ivol(), b, ctx->opt, nullptr, state, b.cs, dt,
+                            ctx->status, s);
     }
-    ctx->launches += 2;
+    ++ctx->launches;
     st = stage == 1 ? ccz4_finish(ctx, sb, stage_state, s)
                     : ccz4_finish(ctx, b, state, s);
     read_diag(ctx, diag);

@@ -766,6 +766,31 @@ __device__ __forceinline__ void block_partial(double v, double *scratch,
 // does not depend on where the z blocks start.
 // One tile (bx, by, bz) of the face pass; `smem_raw` holds faces_smem<T>()
 // bytes; the tile's accretion sum goes to mdot_part[part].
+// With BGK = kGridMetric the geometry comes from a cache of the cells'
+// (launch_ccz4_cells) instead of the background.
+constexpr int kGridMetric = 2;
+
+// Geometry of cell (i,j,k), clamped into the ghosted box, from the cache
+// (gLL[6] gUU[6] lapse shift[3], stride n).
+__device__ __forceinline__ void cached_geo(const double *__restrict__ gc,
+                                           const BoxDev &b, int i, int j,
+                                           int k, Geo &g)
+{
+    const int64_t n = b.gvol();
+    const double *c = gc + b.gidx(min(max(i, b.glo[0]), b.ghi[0]),
+                                  min(max(j, b.glo[1]), b.ghi[1]), k);
+#pragma unroll
+    for (int q = 0; q < 6; ++q)
+        g.gLL[q] = __ldg(&c[q * n]);
+    g.gUU[0] = __ldg(&c[6 * n]);
+    g.gUU[3] = __ldg(&c[9 * n]);
+    g.gUU[5] = __ldg(&c[11 * n]);
+    g.lapse = __ldg(&c[12 * n]);
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+        g.shift[d] = __ldg(&c[(13 + d) * n]);
+}
+
 template <typename T, bool MDOT, bool CG = false, int BGK = -1>
 __device__ __forceinline__ void
 faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
@@ -773,7 +798,7 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
            const Options &o, const FaceOpt<T> &fo, double idx0_, double idx1_,
            double idx2_, int zchunk, int bx, int by, int bz,
            unsigned char *smem_raw, double *__restrict__ mdot_part,
-           int64_t part)
+           int64_t part, const double *__restrict__ gc = nullptr)
 {
     constexpr int nP = kPW * kPW;
     constexpr int nG = kGW * kGW;
@@ -907,9 +932,14 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
                 u = halo < 2 * kTC ? (halo < kTC ? 0 : kGW - 1) : at;
                 v = halo < 2 * kTC ? at : (halo < 3 * kTC ? 0 : kGW - 1);
             }
-            double x, y, z;
-            cell_xyz(o, i0 - 1 + u, j0 - 1 + v, k + 1, x, y, z);
-            metric_T<T, false, BGK>(bg, x, y, z, gn, nullptr);
+            if constexpr (BGK == kGridMetric)
+                cached_geo(gc, b, i0 - 1 + u, j0 - 1 + v, k + 1, gn);
+            else
+            {
+                double x, y, z;
+                cell_xyz(o, i0 - 1 + u, j0 - 1 + v, k + 1, x, y, z);
+                metric_T<T, false, BGK>(bg, x, y, z, gn, nullptr);
+            }
             geo_halve(gn);
             if (pass == 0)
                 geo_store_half(G, nG, v * kGW + u, gn);
@@ -2215,7 +2245,16 @@ __device__ __forceinline__ void ccz4_geo(const double *__restrict__ s,
         geo.shift[d] = s[(kCzShift + d) * cs + g];
 }
 
-// The geometry cache: gLL[6] gUU[6] lapse shift[3] per ghosted cell.
+__device__ __forceinline__ double log_sqrt_det6(const double *g)
+{
+    const double det = g[0] * g[3] * g[5] + 2 * g[1] * g[2] * g[4] -
+                       g[0] * g[4] * g[4] - g[3] * g[2] * g[2] -
+                       g[5] * g[1] * g[1];
+    return (det <= 0.0 || !isfinite(det)) ? 0.0 : 0.5 * log(det);
+}
+
+// The geometry cache: gLL[6] gUU[6] lapse shift[3] ln sqrt(det gamma) per
+// ghosted cell (the sources difference the last along each direction).
 __device__ __forceinline__ void geo_put(double *gc, int64_t n, int64_t g,
                                         const Geo &v)
 {
@@ -2229,6 +2268,7 @@ __device__ __forceinline__ void geo_put(double *gc, int64_t n, int64_t g,
 #pragma unroll
     for (int d = 0; d < 3; ++d)
         gc[(13 + d) * n + g] = v.shift[d];
+    gc[16 * n + g] = log_sqrt_det6(v.gLL);
 }
 
 __device__ __forceinline__ Geo geo_get(const double *__restrict__ gc,
@@ -2248,28 +2288,26 @@ __device__ __forceinline__ Geo geo_get(const double *__restrict__ gc,
     return v;
 }
 
-__device__ __forceinline__ void ghosted_cell(const BoxDev &b, int64_t t,
-                                             int &i, int &j, int &k)
-{
-    const unsigned u = (unsigned)t, nx = b.gn[0], ny = b.gn[1];
-    const unsigned r = u / nx, q = r / ny;
-    i = b.glo[0] + (int)(u - r * nx);
-    j = b.glo[1] + (int)(r - q * ny);
-    k = b.glo[2] + (int)q;
-}
-
 // fill_conserved_outflow_boundaries (:484-519) and
-// fill_ccz4_geometry_outflow_boundaries (:430-473): a physical ghost copies
-// the conserved variables (when `conserved`) and chi, h_ij, lapse, shift of
-// its source cell (the box's end in each direction it lies outside in).
+// fill_ccz4_geometry_outflow_boundaries (:430-473) over the shell of the
+// box: a physical ghost copies the conserved variables q and (with a metric
+// m) chi, h_ij, lapse, shift of its source cell (the box's end in each
+// direction it lies outside in).  With qp, every shell cell also takes its
+// stored primitives from there (a stage state's ghosts hold the state's).
 __global__ void __launch_bounds__(256)
-    k_ccz4_fill(double *__restrict__ s, BoxDev b, int conserved)
+    k_ccz4_fill(double *__restrict__ m, int64_t mcs, double *__restrict__ q,
+                int64_t qcs, const double *__restrict__ qp, int64_t pcs,
+                BoxDev b, int64_t nshell)
 {
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-         t < b.gvol(); t += (int64_t)gridDim.x * blockDim.x)
+         t < nshell; t += (int64_t)gridDim.x * blockDim.x)
     {
         int iv[3];
-        ghosted_cell(b, t, iv[0], iv[1], iv[2]);
+        shell_cell(b, t, iv[0], iv[1], iv[2]);
+        const int64_t g = b.gidx(iv[0], iv[1], iv[2]);
+        if (qp)
+            for (int c = kRho; c < kStateComps; ++c)
+                q[c * qcs + g] = qp[c * pcs + g];
         int src[3] = {iv[0], iv[1], iv[2]};
         bool ghost = false;
 #pragma unroll
@@ -2288,67 +2326,66 @@ __global__ void __launch_bounds__(256)
         }
         if (!ghost)
             continue;
-        const int64_t g = t, sg = b.gidx(src[0], src[1], src[2]);
-        if (conserved)
-            for (int c = 0; c < 5; ++c)
-                s[(kCcz4GrhdOffset + c) * b.cs + g] =
-                    s[(kCcz4GrhdOffset + c) * b.cs + sg];
-        for (int q = 0; q < 7; ++q) // chi, h
-            s[q * b.cs + g] = s[q * b.cs + sg];
-        for (int q = kCzLapse; q < kCzLapse + 4; ++q) // lapse, shift
-            s[q * b.cs + g] = s[q * b.cs + sg];
+        const int64_t sg = b.gidx(src[0], src[1], src[2]);
+        for (int c = 0; c < 5; ++c)
+            q[c * qcs + g] = q[c * qcs + sg];
+        if (!m)
+            continue;
+        for (int c = 0; c < 7; ++c) // chi, h
+            m[c * mcs + g] = m[c * mcs + sg];
+        for (int c = kCzLapse; c < kCzLapse + 4; ++c) // lapse, shift
+            m[c * mcs + g] = m[c * mcs + sg];
     }
 }
 
 // recover_primitives_from_ccz4_geometry over the ghosted box (:681-702):
-// the primitive cache (rho, p, v) and the geometry cache of every cell.
+// the primitive cache (rho, p, v) and, unless it holds this metric already
+// (fresh = 0), the geometry cache of every cell.
 __global__ void __launch_bounds__(256)
-    k_ccz4_cells(const double *__restrict__ s, BoxDev b, Options o,
-                 double *__restrict__ prim, double *__restrict__ gc,
-                 DevStatus *st)
+    k_ccz4_cells(const double *__restrict__ m, int64_t mcs,
+                 const double *__restrict__ q, int64_t qcs, BoxDev b,
+                 Options o, double *__restrict__ prim,
+                 double *__restrict__ gc, int fresh, DevStatus *st)
 {
-    const double *q = s + kCcz4GrhdOffset * b.cs;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-         t < b.gvol(); t += (int64_t)gridDim.x * blockDim.x)
+    const int64_t n = b.gvol();
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
+         t += (int64_t)gridDim.x * blockDim.x)
     {
         Geo geo;
-        ccz4_geo(s, b.cs, t, geo, nullptr);
-        geo_put(gc, b.gvol(), t, geo);
+        if (fresh)
+        {
+            ccz4_geo(m, mcs, t, geo, nullptr);
+            geo_put(gc, n, t, geo);
+        }
+        else
+        {
+#pragma unroll
+            for (int c = 0; c < 6; ++c)
+                geo.gUU[c] = gc[(6 + c) * n + t];
+        }
         Prim pr;
-        if (!con2prim(o, load_cons(q, b.cs, t), geo.gUU, pr, nullptr,
-                      nullptr))
+        if (!con2prim(o, load_cons(q, qcs, t), geo.gUU, pr, nullptr, nullptr))
         {
             record_error(st, 2, t);
             pr.rho = pr.p = 1.0;
             pr.v[0] = pr.v[1] = pr.v[2] = 0.0;
         }
-        store_pv(prim, b.gvol(), t, pr);
+        store_pv(prim, n, t, pr);
     }
 }
 
-__device__ __forceinline__ double log_sqrt_det6(const double *g)
-{
-    const double det = g[0] * g[3] * g[5] + 2 * g[1] * g[2] * g[4] -
-                       g[0] * g[4] * g[4] - g[3] * g[2] * g[2] -
-                       g[5] * g[1] * g[1];
-    return (det <= 0.0 || !isfinite(det)) ? 0.0 : 0.5 * log(det);
-}
-
-// The RHS of one interior cell: per direction the two faces of the cell
-// (compute_directional_flux_rhs_from_ccz4_geometry, :784-833, every face
-// twice as the reference computes it), then the static-metric sources with
-// finite-difference derivatives (add_static_metric_sources_to_conserved_rhs,
-// :367-427; one-sided where a neighbour's stored primitives are metric-
-// source atmosphere, make_metric_source_derivative_stencil, :283-322).
-__global__ void __launch_bounds__(256, 2)
-    k_ccz4_rhs(const double *__restrict__ s, BoxDev b, Options o,
-               FaceOpt<double> fo,
+// The static-metric sources of an interior cell with finite-difference
+// derivatives (add_static_metric_sources_to_conserved_rhs, :367-427;
+// one-sided where a neighbour's stored primitives are metric-source
+// atmosphere, make_metric_source_derivative_stencil, :283-322).
+__global__ void __launch_bounds__(256, 3)
+    k_ccz4_src(const double *__restrict__ m, int64_t mcs,
+               const double *__restrict__ q, int64_t qcs, BoxDev b, Options o,
                const double *__restrict__ prim, const double *__restrict__ gc,
-               double *__restrict__ rhs, int64_t rcs, double inv0,
-               double inv1, double inv2, DevStatus *st)
+               double *__restrict__ src, double inv0, double inv1,
+               double inv2)
 {
     const int64_t n = b.gvol();
-    const double *q = s + kCcz4GrhdOffset * b.cs;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
          t < b.ivol(); t += (int64_t)gridDim.x * blockDim.x)
     {
@@ -2358,108 +2395,160 @@ __global__ void __launch_bounds__(256, 2)
         const double inv[3] = {inv0, inv1, inv2};
         const int64_t step[3] = {1, (int64_t)b.gn[0],
                                  (int64_t)b.gn[0] * b.gn[1]};
-        Cons r;
-        r.D = r.tau = 0.0;
-        r.S[0] = r.S[1] = r.S[2] = 0.0;
-        for (int d = 0; d < 3; ++d)
+        Cons s = zero_cons<double>();
+        const Geo ge = geo_get(gc, n, g);
+        const PV pv = load_pv_global<double>(prim, n, g);
+        Prim pr;
+        pr.rho = pv.q[0];
+        pr.p = pv.q[1];
+        pr.v[0] = pv.q[2];
+        pr.v[1] = pv.q[3];
+        pr.v[2] = pv.q[4];
+        floors(o, pr, ge.gLL);
+        if (o.use_src && !is_atmo(o, pr, o.src_atmo_factor))
         {
-            const int64_t so = step[d];
-            Cons f[2];
-            for (int side = 0; side < 2; ++side)
+            // compute_static_metric_source_terms (static_sources), one
+            // direction's derivatives at a time
+            const Cons c = load_cons(q, qcs, g);
+            const double W = rsqrt_(1.0 - vsq(pr.v, ge.gLL));
+            const double h = 1.0 + pr.eps + div_(pr.p, pr.rho);
+            const double rhw = pr.rho * h * W * W;
+            double T[6], mU[3];
+#pragma unroll
+            for (int e = 0; e < 3; ++e)
+#pragma unroll
+                for (int f = e; f < 3; ++f)
+                    T[sym(e, f)] = rhw * pr.v[e] * pr.v[f] +
+                                   pr.p * ge.gUU[sym(e, f)];
+            raise(ge.gUU, c.S, mU);
+            const double E = c.D + c.tau;
             {
-                const int64_t L = g - so + side * so, R = L + so;
-                Geo gf;
-                average_geo(geo_get(gc, n, L), geo_get(gc, n, R), gf);
-                f[side] = face_flux(fo, load_pv_global<double>(prim, n, L - so),
-                                    load_pv_global<double>(prim, n, L),
-                                    load_pv_global<double>(prim, n, R),
-                                    load_pv_global<double>(prim, n, R + so),
-                                    gf, d);
+                const double ichi = 1.0 / m[kCzChi * mcs + g];
+                const double tr3 = m[kCzK * mcs + g] / 3.0;
+                double sk = 0.0;
+#pragma unroll
+                for (int e = 0; e < 3; ++e)
+#pragma unroll
+                    for (int f = e; f < 3; ++f)
+                    {
+                        const int a = sym(e, f);
+                        const double K =
+                            m[(kCzA + a) * mcs + g] * ichi + ge.gLL[a] * tr3;
+                        sk += (e == f ? 1.0 : 2.0) * T[a] * K;
+                    }
+                s.tau = ge.lapse * sk;
             }
-            r.D += -inv[d] * (f[1].D - f[0].D);
-            r.tau += -inv[d] * (f[1].tau - f[0].tau);
 #pragma unroll
-            for (int m = 0; m < 3; ++m)
-                r.S[m] += -inv[d] * (f[1].S[m] - f[0].S[m]);
-        }
-        if (o.use_src)
-        {
-            GeoFull fg;
-            ccz4_geo(s, b.cs, g, fg.g, fg.K);
-            const PV pv = load_pv_global<double>(prim, n, g);
-            Prim pr;
-            pr.rho = pv.q[0];
-            pr.p = pv.q[1];
-            pr.v[0] = pv.q[2];
-            pr.v[1] = pv.q[3];
-            pr.v[2] = pv.q[4];
-            floors(o, pr, fg.g.gLL);
-            if (!is_atmo(o, pr, o.src_atmo_factor))
+            for (int d = 0; d < 3; ++d)
             {
-                for (int d = 0; d < 3; ++d)
-                {
-                    fg.dlapse[d] = fg.dlnsqrtg[d] = 0.0;
+                const int64_t lo_i = g - step[d], hi_i = g + step[d];
+                Prim pl, pu;
+                pl.rho = q[kRho * qcs + lo_i];
+                pl.p = q[kPress * qcs + lo_i];
+                pu.rho = q[kRho * qcs + hi_i];
+                pu.p = q[kPress * qcs + hi_i];
+                const bool la = !is_atmo(o, pl, o.src_atmo_factor);
+                const bool ua = !is_atmo(o, pu, o.src_atmo_factor);
+                // no fluid neighbour: zero derivatives
+                const int64_t lc = la ? lo_i : g, uc = ua ? hi_i : g;
+                const double coef = la && ua ? 0.5 * inv[d]
+                                    : la || ua ? inv[d]
+                                               : 0.0;
+                const auto diff = [&](int field) {
+                    return coef *
+                           (gc[field * n + uc] - gc[field * n + lc]);
+                };
+                const double dlapse = diff(12), dlns = diff(16);
+                double ms = -E * dlapse, sg = 0.0;
 #pragma unroll
-                    for (int q6 = 0; q6 < 6; ++q6)
-                        fg.dgamma[d][q6] = 0.0;
+                for (int e = 0; e < 3; ++e)
 #pragma unroll
-                    for (int m = 0; m < 3; ++m)
-                        fg.dshift[m][d] = 0.0;
-                    const int64_t lo_i = g - step[d], hi_i = g + step[d];
-                    Prim pl, pu;
-                    pl.rho = q[kRho * b.cs + lo_i];
-                    pl.p = q[kPress * b.cs + lo_i];
-                    pu.rho = q[kRho * b.cs + hi_i];
-                    pu.p = q[kPress * b.cs + hi_i];
-                    const bool la = !is_atmo(o, pl, o.src_atmo_factor);
-                    const bool ua = !is_atmo(o, pu, o.src_atmo_factor);
-                    int64_t lc, uc;
-                    double coef;
-                    if (la && ua)
-                    {
-                        lc = lo_i;
-                        uc = hi_i;
-                        coef = 0.5 * inv[d];
-                    }
-                    else if (ua)
-                    {
-                        lc = g;
-                        uc = hi_i;
-                        coef = inv[d];
-                    }
-                    else if (la)
-                    {
-                        lc = lo_i;
-                        uc = g;
-                        coef = inv[d];
-                    }
-                    else
-                        continue;
-                    const Geo gu = geo_get(gc, n, uc), gl = geo_get(gc, n, lc);
-                    fg.dlapse[d] = coef * (gu.lapse - gl.lapse);
-                    fg.dlnsqrtg[d] =
-                        coef * (log_sqrt_det6(gu.gLL) - log_sqrt_det6(gl.gLL));
+                    for (int f = e; f < 3; ++f)
+                        sg += (e == f ? 1.0 : 2.0) * T[sym(e, f)] *
+                              diff(sym(e, f));
+                ms += 0.5 * ge.lapse * sg;
 #pragma unroll
-                    for (int q6 = 0; q6 < 6; ++q6)
-                        fg.dgamma[d][q6] = coef * (gu.gLL[q6] - gl.gLL[q6]);
+                for (int e = 0; e < 3; ++e)
+                    ms += c.S[e] * diff(13 + e);
+                const Cons F = phys_flux(pr, c, d, ge.lapse, ge.shift);
+                s.S[d] += ms;
+                s.D -= F.D * dlns;
+                s.tau -= F.tau * dlns + mU[d] * dlapse;
 #pragma unroll
-                    for (int m = 0; m < 3; ++m)
-                        fg.dshift[m][d] = coef * (gu.shift[m] - gl.shift[m]);
-                }
-                const Cons c = load_cons(q, b.cs, g);
-                const Cons src = static_sources(pr, c, fg);
-                r.D += src.D;
-                r.tau += src.tau;
-#pragma unroll
-                for (int m = 0; m < 3; ++m)
-                    r.S[m] += src.S[m];
+                for (int e = 0; e < 3; ++e)
+                    s.S[e] -= F.S[e] * dlns;
             }
         }
-        rhs[0 * rcs + t] = r.D;
-        rhs[1 * rcs + t] = r.S[0];
-        rhs[2 * rcs + t] = r.S[1];
-        rhs[3 * rcs + t] = r.S[2];
-        rhs[4 * rcs + t] = r.tau;
+        store_src(src, b.rcs, t, s);
+    }
+}
+
+// The flux differences and sources of the RHS
+// (compute_directional_flux_rhs_from_ccz4_geometry, :784-833): the face pass
+// with its geometry from the cache.  One thread per cell evaluating the
+// cell's six faces (each face twice, as the reference does) took 254 us at
+// 100 x 90 x 70; this and k_ccz4_src take 190.
+__global__ void __launch_bounds__(kTB *kTB, 2)
+    k_ccz4_faces(const double *__restrict__ prim,
+                 const double *__restrict__ src, double *__restrict__ rhs,
+                 BoxDev b, Options o, FaceOpt<double> fo, double idx0,
+                 double idx1, double idx2, int zchunk,
+                 const double *__restrict__ gc)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    faces_tile<double, false, false, kGridMetric>(
+        prim, src, rhs, b, Background(), o, fo, idx0, idx1, idx2, zchunk,
+        blockIdx.x, blockIdx.y, blockIdx.z, smem_raw, nullptr, 0, gc);
+}
+
+// One stage of an integrator fused with the recovery: out = in + dt rhs, or
+// with u1 the SSPRK2 combination out = (in + u1 + dt rhs) / 2
+// (add_scaled_conserved_rhs, :927-940, combine_ssprk2_conserved_state,
+// :942-969), then recover_primitives_and_apply_atmosphere_from_ccz4_geometry
+// (:713-761) on the cached geometry or (gc null) that of the metric m.  GRHD
+// components, FP64.
+__global__ void __launch_bounds__(256)
+    k_ccz4_advance(double *out, int64_t ocs, const double *in, int64_t ics,
+                   const double *u1, int64_t ucs,
+                   const double *__restrict__ rhs, int64_t rcs, BoxDev b,
+                   Options o, const double *__restrict__ gc,
+                   const double *__restrict__ m, int64_t mcs, double dt,
+                   DevStatus *st)
+{
+    unsigned long long cnt[4] = {0, 0, 0, 0};
+    const int64_t n = b.ivol();
+    const int64_t n_pad = (n + blockDim.x - 1) / blockDim.x * blockDim.x;
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n_pad;
+         t += (int64_t)gridDim.x * blockDim.x)
+    {
+        if (t < n)
+        {
+            int i, j, k;
+            interior_cell(b, t, i, j, k);
+            const int64_t g = b.gidx(i, j, k);
+            double u[5];
+#pragma unroll
+            for (int c = 0; c < 5; ++c)
+            {
+                const double x = rhs[c * rcs + t], u0 = in[c * ics + g];
+                u[c] = u1 ? 0.5 * (u0 + u1[c * ucs + g] + dt * x)
+                          : u0 + dt * x;
+            }
+            Cons c;
+            c.D = u[0];
+            c.S[0] = u[1];
+            c.S[1] = u[2];
+            c.S[2] = u[3];
+            c.tau = u[4];
+            Geo geo;
+            if (gc)
+                geo = geo_get(gc, b.gvol(), g);
+            else
+                ccz4_geo(m, mcs, g, geo, nullptr);
+            recover_cell<double>(o, geo, c, out, ocs, g, cnt);
+        }
+        flush_counts(st, cnt);
+        cnt[0] = cnt[1] = cnt[2] = cnt[3] = 0;
     }
 }
 
@@ -2531,16 +2620,12 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// add_scaled_conserved_rhs (:927-940) and combine_ssprk2_conserved_state
-// (:942-969) on the GRHD components: mode 0 s += dt rhs; mode 1
-// s = (s + u1 + dt rhs) / 2.
+// add_scaled_conserved_rhs (:927-940) on the GRHD components: s += dt rhs.
 __global__ void __launch_bounds__(256)
-    k_ccz4_update(double *__restrict__ s, const double *__restrict__ u1,
-                  int64_t ucs, const double *__restrict__ rhs, int64_t rcs,
-                  BoxDev b, double dt, int mode)
+    k_ccz4_update(double *__restrict__ s, const double *__restrict__ rhs,
+                  int64_t rcs, BoxDev b, double dt)
 {
     double *q = s + kCcz4GrhdOffset * b.cs;
-    const double *u = u1 ? u1 + kCcz4GrhdOffset * ucs : nullptr;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
          t < b.ivol(); t += (int64_t)gridDim.x * blockDim.x)
     {
@@ -2548,14 +2633,7 @@ __global__ void __launch_bounds__(256)
         interior_cell(b, t, i, j, k);
         const int64_t g = b.gidx(i, j, k);
         for (int c = 0; c < 5; ++c)
-        {
-            const double x = rhs[c * rcs + t];
-            if (mode == 0)
-                q[c * b.cs + g] += dt * x;
-            else
-                q[c * b.cs + g] = 0.5 * (q[c * b.cs + g] + u[c * ucs + g] +
-                                         dt * x);
-        }
+            q[c * b.cs + g] += dt * rhs[c * rcs + t];
     }
 }
 
@@ -2593,6 +2671,8 @@ cudaError_t configure_kernels()
     for (const void *k : fp32)
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(k, attr, f);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_ccz4_faces, attr, d);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_ensemble<double>, attr,
                                  (int)faces_smem<double>());
@@ -2980,29 +3060,52 @@ void launch_eval_arith(int64_t n, const double *a, const double *b,
     k_eval_arith<<<(int)((n + 255) / 256), 256, 0, s>>>(n, a, b, out);
 }
 
-void launch_ccz4_fill(double *s, const BoxDev &b, bool conserved,
+void launch_ccz4_fill(double *m, int64_t mcs, double *q, int64_t qcs,
+                      const double *qp, int64_t pcs, const BoxDev &b,
                       cudaStream_t st)
 {
-    k_ccz4_fill<<<grid_for(b.gvol(), 256), 256, 0, st>>>(s, b,
-                                                          conserved ? 1 : 0);
+    const int64_t nshell = b.gvol() - b.ivol();
+    if (nshell > 0)
+        k_ccz4_fill<<<grid_for(nshell, 256), 256, 0, st>>>(m, mcs, q, qcs, qp,
+                                                           pcs, b, nshell);
 }
 
-void launch_ccz4_cells(const double *s, const BoxDev &b, const Options &o,
-                       double *prim, double *gc, DevStatus *st,
+void launch_ccz4_cells(const double *m, int64_t mcs, const double *q,
+                       int64_t qcs, const BoxDev &b, const Options &o,
+                       double *prim, double *gc, bool fresh, DevStatus *st,
                        cudaStream_t stream)
 {
-    k_ccz4_cells<<<grid_for(b.gvol(), 256), 256, 0, stream>>>(s, b, o, prim,
-                                                               gc, st);
+    k_ccz4_cells<<<grid_for(b.gvol(), 256), 256, 0, stream>>>(
+        m, mcs, q, qcs, b, o, prim, gc, fresh ? 1 : 0, st);
 }
 
-void launch_ccz4_rhs(const double *s, const BoxDev &b, const Options &o,
-                     const double *prim, const double *gc, double *rhs,
-                     int64_t rcs, const double inv[3], DevStatus *st,
-                     cudaStream_t stream)
+void launch_ccz4_rhs(const double *m, int64_t mcs, const double *q,
+                     int64_t qcs, const BoxDev &b, const Options &o,
+                     const double *prim, const double *gc, double *src,
+                     double *rhs, const double inv[3], cudaStream_t stream)
 {
-    k_ccz4_rhs<<<grid_for(b.ivol(), 256), 256, 0, stream>>>(
-        s, b, o, make_face_opt<double>(o), prim, gc, rhs, rcs, inv[0], inv[1],
-        inv[2], st);
+    k_ccz4_src<<<grid_for(b.ivol(), 256), 256, 0, stream>>>(
+        m, mcs, q, qcs, b, o, prim, gc, src, inv[0], inv[1], inv[2]);
+    const int zchunk = face_zchunk(b, 0, false);
+    const dim3 grid((b.in[0] + kTC - 1) / kTC, (b.in[1] + kTC - 1) / kTC,
+                    (b.in[2] + zchunk - 1) / zchunk);
+    // this operator has no excision
+    Options of = o;
+    of.excision_radius = 0.0;
+    k_ccz4_faces<<<grid, dim3(kTB, kTB), faces_smem<double>(), stream>>>(
+        prim, src, rhs, b, of, make_face_opt<double>(o), inv[0], inv[1],
+        inv[2], zchunk, gc);
+}
+
+void launch_ccz4_advance(double *out, int64_t ocs, const double *in,
+                         int64_t ics, const double *u1, int64_t ucs,
+                         const double *rhs, int64_t rcs, const BoxDev &b,
+                         const Options &o, const double *gc, const double *m,
+                         int64_t mcs, double dt, DevStatus *st,
+                         cudaStream_t stream)
+{
+    k_ccz4_advance<<<grid_for(b.ivol(), 256), 256, 0, stream>>>(
+        out, ocs, in, ics, u1, ucs, rhs, rcs, b, o, gc, m, mcs, dt, st);
 }
 
 void launch_ccz4_recover(double *s, const BoxDev &b, const Options &o,
@@ -3019,12 +3122,11 @@ void launch_ccz4_max_inv_dt(const double *s, const BoxDev &b,
         s, b, o, inv[0], inv[1], inv[2], st);
 }
 
-void launch_ccz4_update(double *s, const double *u1, int64_t ucs,
-                        const double *rhs, int64_t rcs, const BoxDev &b,
-                        double dt, int mode, cudaStream_t stream)
+void launch_ccz4_update(double *s, const double *rhs, int64_t rcs,
+                        const BoxDev &b, double dt, cudaStream_t stream)
 {
-    k_ccz4_update<<<grid_for(b.ivol(), 256), 256, 0, stream>>>(
-        s, u1, ucs, rhs, rcs, b, dt, mode);
+    k_ccz4_update<<<grid_for(b.ivol(), 256), 256, 0, stream>>>(s, rhs, rcs, b,
+                                                                dt);
 }
 
 void launch_ccz4_probe(const double *s, const BoxDev &b, const Options &o,

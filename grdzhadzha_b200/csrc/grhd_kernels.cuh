@@ -294,26 +294,38 @@ template <typename T> cudaError_t ensemble_occupancy(int *blocks_per_sm);
 template <typename T>
 cudaError_t launch_ensemble(const EnsLaunch &a, int grid, cudaStream_t s);
 
-// The operator on CCZ4-stored geometry (grhd_kernels.cu): state of 36
-// components (25 CCZ4, then 11 GRHD), stride b.cs; the geometry cache holds
-// gLL[6] gUU[6] lapse shift[3] over the ghosted box.
-void launch_ccz4_fill(double *s, const BoxDev &b, bool conserved,
+constexpr int kCcz4GeoFields = 17;
+// The operator on CCZ4-stored geometry (grhd_kernels.cu): a state of 36
+// components, 25 CCZ4 ones (m, stride mcs) then 11 GRHD ones (q, stride qcs);
+// the geometry cache gc holds gLL[6] gUU[6] lapse shift[3] ln sqrt(gamma)
+// (kCcz4GeoFields) over the ghosted box.  A null m leaves the metric's ghosts, fresh = false the cache.
+void launch_ccz4_fill(double *m, int64_t mcs, double *q, int64_t qcs,
+                      const double *qp, int64_t pcs, const BoxDev &b,
                       cudaStream_t st);
-void launch_ccz4_cells(const double *s, const BoxDev &b, const Options &o,
-                       double *prim, double *gc, DevStatus *st,
+void launch_ccz4_cells(const double *m, int64_t mcs, const double *q,
+                       int64_t qcs, const BoxDev &b, const Options &o,
+                       double *prim, double *gc, bool fresh, DevStatus *st,
                        cudaStream_t stream);
-void launch_ccz4_rhs(const double *s, const BoxDev &b, const Options &o,
-                     const double *prim, const double *gc, double *rhs,
-                     int64_t rcs, const double inv[3], DevStatus *st,
-                     cudaStream_t stream);
+// rhs and the source scratch have stride b.rcs.
+void launch_ccz4_rhs(const double *m, int64_t mcs, const double *q,
+                     int64_t qcs, const BoxDev &b, const Options &o,
+                     const double *prim, const double *gc, double *src,
+                     double *rhs, const double inv[3], cudaStream_t stream);
+// out = in + dt rhs, or (in + u1 + dt rhs) / 2 with u1, then the recovery on
+// the cached geometry or, with gc null, that of the metric m.
+void launch_ccz4_advance(double *out, int64_t ocs, const double *in,
+                         int64_t ics, const double *u1, int64_t ucs,
+                         const double *rhs, int64_t rcs, const BoxDev &b,
+                         const Options &o, const double *gc, const double *m,
+                         int64_t mcs, double dt, DevStatus *st,
+                         cudaStream_t stream);
 void launch_ccz4_recover(double *s, const BoxDev &b, const Options &o,
                          DevStatus *st, cudaStream_t stream);
 void launch_ccz4_max_inv_dt(const double *s, const BoxDev &b,
                             const Options &o, const double inv[3],
                             DevStatus *st, cudaStream_t stream);
-void launch_ccz4_update(double *s, const double *u1, int64_t ucs,
-                        const double *rhs, int64_t rcs, const BoxDev &b,
-                        double dt, int mode, cudaStream_t stream);
+void launch_ccz4_update(double *s, const double *rhs, int64_t rcs,
+                        const BoxDev &b, double dt, cudaStream_t stream);
 void launch_ccz4_probe(const double *s, const BoxDev &b, const Options &o,
                        int i, int j, int k, double *out, cudaStream_t stream);
 
