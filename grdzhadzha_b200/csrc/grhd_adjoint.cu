@@ -97,9 +97,12 @@ __global__ void __launch_bounds__(256)
                         t);
 }
 
-// three resident blocks per SM (168 registers, small spills)
+// One direction's faces.  The direction is a template parameter: as a run-time
+// value it indexes the geometry, shift and momentum arrays, which then live
+// in local memory (800 bytes a thread; 61 us per launch at 64^3, 32 so).
+template <int d>
 __global__ void __launch_bounds__(kAdjThreads, 3)
-    k_adj_faces(AdjRhs A, int d, double *slot)
+    k_adj_faces(AdjRhs A, double *slot)
 {
     int n[3] = {A.b.in[0], A.b.in[1], A.b.in[2]};
     n[d] += 1;
@@ -113,15 +116,23 @@ __global__ void __launch_bounds__(kAdjThreads, 3)
 
 __global__ void __launch_bounds__(256) k_adj_shell(AdjRhs A, double *slot)
 {
-    const int64_t n = A.b.gvol();
+    const int k0 = A.b.glo[2], k1 = A.b.ghi[2];
+    const int64_t n = plane_shell_count(A.b, k0, k1);
     double spin = 0.0;
-    for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < n;
-         g += (int64_t)gridDim.x * blockDim.x)
-        spin += shell_rev_item(A, g);
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
+         t += (int64_t)gridDim.x * blockDim.x)
+    {
+        int i, j, k;
+        plane_shell_cell(A.b, k0, k1, t, i, j, k);
+        spin += shell_rev_item(A, A.b.gidx(i, j, k));
+    }
     block_add(spin, slot);
 }
 
-__global__ void __launch_bounds__(kAdjThreads)
+// Three resident blocks (168 registers): with the sources' metric adjoint no
+// longer formed, they cost less in spills than they hide (per 64^3 gradient
+// of four steps 7.6 ms with two, 7.1 with three).
+__global__ void __launch_bounds__(kAdjThreads, 3)
     k_adj_cells(AdjRhs A, AdjStage S, double *slot)
 {
     const int64_t n = A.b.ivol();
@@ -364,9 +375,10 @@ void reverse_rhs(grhd_adjoint *a, const grhd_adjoint::Slot &sl, int st,
                  double mu, const AdjStage &S, cudaStream_t s)
 {
     const AdjRhs A = rhs_args(a, sl, st, mu);
-    for (int d = 0; d < 3; ++d)
-        k_adj_faces<<<a->grid, kAdjThreads, 0, s>>>(
-            A, d, a->spin_slots + (int64_t)d * a->grid);
+    k_adj_faces<0><<<a->grid, kAdjThreads, 0, s>>>(A, a->spin_slots);
+    k_adj_faces<1><<<a->grid, kAdjThreads, 0, s>>>(A, a->spin_slots + a->grid);
+    k_adj_faces<2><<<a->grid, kAdjThreads, 0, s>>>(
+        A, a->spin_slots + (int64_t)2 * a->grid);
     k_adj_shell<<<a->grid, 256, 0, s>>>(A, a->spin_slots +
                                                (int64_t)3 * a->grid);
     k_adj_cells<<<a->grid, kAdjThreads, 0, s>>>(

@@ -105,14 +105,15 @@ GRHD_HD inline void vsq_rev(const double v[3], const double G[6],
 }
 
 // compute_conserved (p2c), Valencia.hpp:55-73
-GRHD_HD inline void p2c_rev(const Prim &pr, const double G[6],
+GRHD_HD __forceinline__ void p2c_rev(const Prim &pr, const double G[6],
                             const ConsBar &cb, PrimBar &pb, double Gbar[6])
 {
     double vL[3];
     lower(G, pr.v, vL);
     const double v2 = vL[0] * pr.v[0] + vL[1] * pr.v[1] + vL[2] * pr.v[2];
-    const double W = 1.0 / sqrt(1.0 - v2);
-    const double h = 1.0 + pr.eps + pr.p / pr.rho;
+    const double W = rsqrt_ulp(1.0 - v2);
+    const double irho = rcp_ulp(pr.rho), y = pr.p * irho;
+    const double h = 1.0 + pr.eps + y;
     const double rhw = pr.rho * h * W * W;
     const double rhwbar =
         cb.tau + cb.S[0] * vL[0] + cb.S[1] * vL[1] + cb.S[2] * vL[2];
@@ -127,8 +128,8 @@ GRHD_HD inline void p2c_rev(const Prim &pr, const double G[6],
     const double hbar = rhwbar * pr.rho * W * W;
     Wbar += rhwbar * pr.rho * h * 2.0 * W;
     pb.eps += hbar;
-    pb.p += hbar / pr.rho;
-    pb.rho -= hbar * pr.p / (pr.rho * pr.rho);
+    pb.p += hbar * irho;
+    pb.rho -= hbar * y * irho;
     const double v2bar = Wbar * 0.5 * W * W * W;
     // vL = G v
     double t[3];
@@ -142,7 +143,7 @@ GRHD_HD inline void p2c_rev(const Prim &pr, const double G[6],
 // enforce_primitive_floors, Atmosphere.hpp:24-46.  `in` is the input of
 // the floors (eps unused: the floors recompute it); `ob` the adjoint of
 // their output (eps included); adds the adjoint of rho, p, v of the input.
-GRHD_HD inline void floors_rev(const Options &o, const Prim &in,
+GRHD_HD __forceinline__ void floors_rev(const Options &o, const Prim &in,
                                const double G[6], const PrimBar &ob,
                                PrimBar &ib, double Gbar[6])
 {
@@ -150,8 +151,9 @@ GRHD_HD inline void floors_rev(const Options &o, const Prim &in,
     const double p1 = fmax(in.p, o.p_floor);
     const double gm1 = o.G - 1.0;
     double rho1bar = ob.rho, p1bar = ob.p;
-    p1bar += ob.eps / (gm1 * rho1);
-    rho1bar -= ob.eps * p1 / (gm1 * rho1 * rho1);
+    const double ir = rcp_ulp(rho1), epsbar = ob.eps * rcp_ulp(gm1) * ir;
+    p1bar += epsbar;
+    rho1bar -= epsbar * p1 * ir;
     if (in.rho > o.rho_floor)
         ib.rho += rho1bar;
     if (in.p > o.p_floor)
@@ -159,12 +161,12 @@ GRHD_HD inline void floors_rev(const Options &o, const Prim &in,
     const double v2 = vsq(in.v, G);
     if (v2 >= o.atmo_vmax2)
     {
-        const double s = sqrt(o.atmo_vmax2 / v2);
+        const double s = sqrt_(div_(o.atmo_vmax2, v2));
         const double sbar =
             ob.v[0] * in.v[0] + ob.v[1] * in.v[1] + ob.v[2] * in.v[2];
         for (int k = 0; k < 3; ++k)
             ib.v[k] += s * ob.v[k];
-        vsq_rev(in.v, G, -0.5 * s / v2 * sbar, ib.v, Gbar);
+        vsq_rev(in.v, G, div_(-0.5 * s, v2) * sbar, ib.v, Gbar);
     }
     else
     {
@@ -174,7 +176,7 @@ GRHD_HD inline void floors_rev(const Options &o, const Prim &in,
 }
 
 // compute_flux, Valencia.hpp:230-259
-GRHD_HD inline void phys_flux_rev(const Prim &pr, const Cons &c, int d,
+GRHD_HD __forceinline__ void phys_flux_rev(const Prim &pr, const Cons &c, int d,
                                   double lapse, const double shift[3],
                                   const ConsBar &fb, PrimBar &pb, ConsBar &cb,
                                   double &lapse_bar, double shift_bar[3])
@@ -195,23 +197,25 @@ GRHD_HD inline void phys_flux_rev(const Prim &pr, const Cons &c, int d,
 }
 
 // compute_characteristic_speeds (shifted), RiemannSolvers.hpp:23-67
-GRHD_HD inline void char_speeds_rev(const Options &o, const Prim &pr,
+GRHD_HD __forceinline__ void char_speeds_rev(const Options &o, const Prim &pr,
                                     const Geo &g, int d, double lobar,
                                     double hibar, PrimBar &pb, GeoBar &gb)
 {
     const double v2 = vsq(pr.v, g.gLL);
-    const double h = 1.0 + pr.eps + pr.p / pr.rho;
-    const double cs2 = o.G * pr.p / (pr.rho * h);
-    const double cs = sqrt(cs2);
+    const double irho = rcp_ulp(pr.rho), y = pr.p * irho;
+    const double h = 1.0 + pr.eps + y;
+    const double ih = rcp_ulp(h);
+    const double cs2 = o.G * y * ih;
+    const double ics = rsqrt_ulp(cs2), cs = cs2 * ics;
     const double vel = pr.v[d];
     const double den = 1.0 - v2 * cs2;
     const double gdd = g.gUU[sym(d, d)];
     const double Q = gdd * den - vel * vel * (1.0 - cs2);
     const double rad = (1.0 - v2) * Q;
-    const double sr = sqrt(fmax(0.0, rad));
+    const double isr = rad > 0.0 ? rsqrt_ulp(rad) : 0.0, sr = rad * isr;
     const double root = cs * sr;
     const double base = vel * (1.0 - cs2);
-    const double iden = 1.0 / den;
+    const double iden = rcp_ulp(den);
 
     gb.shift[d] -= lobar + hibar;
     gb.lapse += lobar * (base - root) * iden + hibar * (base + root) * iden;
@@ -223,7 +227,7 @@ GRHD_HD inline void char_speeds_rev(const Options &o, const Prim &pr,
     double velbar = basebar * (1.0 - cs2);
     double cs2bar = -basebar * vel;
     double csbar = rootbar * sr;
-    double radbar = (rad > 0.0) ? rootbar * cs / (2.0 * sr) : 0.0;
+    double radbar = rootbar * cs * 0.5 * isr;
     double v2bar = -radbar * Q;
     const double Qbar = radbar * (1.0 - v2);
     gb.gUU[sym(d, d)] += Qbar * den;
@@ -232,14 +236,14 @@ GRHD_HD inline void char_speeds_rev(const Options &o, const Prim &pr,
     cs2bar += Qbar * vel * vel;
     v2bar -= denbar * cs2;
     cs2bar -= denbar * v2;
-    cs2bar += csbar / (2.0 * cs);
+    cs2bar += csbar * 0.5 * ics;
     // cs2 = G p / (rho h)
-    pb.p += cs2bar * o.G / (pr.rho * h);
-    pb.rho -= cs2bar * cs2 / pr.rho;
-    const double hbar = -cs2bar * cs2 / h;
+    pb.p += cs2bar * o.G * irho * ih;
+    pb.rho -= cs2bar * cs2 * irho;
+    const double hbar = -cs2bar * cs2 * ih;
     pb.eps += hbar;
-    pb.p += hbar / pr.rho;
-    pb.rho -= hbar * pr.p / (pr.rho * pr.rho);
+    pb.p += hbar * irho;
+    pb.rho -= hbar * y * irho;
     pb.v[d] += velbar;
     vsq_rev(pr.v, g.gLL, v2bar, pb.v, gb.gLL);
 }
@@ -336,7 +340,7 @@ GRHD_HD inline int bits_of(unsigned bits, int q) { return (bits >> (2 * q)) & 3;
 // the floors (qlbar, qrbar, rho p v order) and adds the face-geometry
 // adjoint.  Returns F_D (the forward rest-mass flux) for the accretion
 // term.
-GRHD_HD inline double face_flux_rev(const Options &o, const double LL[5],
+GRHD_HD __forceinline__ double face_flux_rev(const Options &o, const double LL[5],
                                     const double L[5], const double R[5],
                                     const double RR[5], unsigned bitsL,
                                     unsigned bitsR, const Geo &g, int d,
@@ -401,7 +405,7 @@ GRHD_HD inline double face_flux_rev(const Options &o, const double LL[5],
     }
     else
     {
-        const double inv = 1.0 / (su - sl);
+        const double inv = rcp_ulp(su - sl);
         const double ss = sl * su;
         const double lfv[5] = {lf.D, lf.S[0], lf.S[1], lf.S[2], lf.tau};
         const double rfv[5] = {rf.D, rf.S[0], rf.S[1], rf.S[2], rf.tau};
@@ -452,26 +456,40 @@ GRHD_HD inline double face_flux_rev(const Options &o, const double LL[5],
         else
             rhib = subar;
     }
-    PrimBar lpb = zero_prim_bar(), rpb = zero_prim_bar();
-    phys_flux_rev(lp, lc, d, g.lapse, g.shift, lfb, lpb, lcb, gb.lapse,
-                  gb.shift);
-    phys_flux_rev(rp, rc, d, g.lapse, g.shift, rfb, rpb, rcb, gb.lapse,
-                  gb.shift);
-    char_speeds_rev(o, lp, g, d, llob, lhib, lpb, gb);
-    char_speeds_rev(o, rp, g, d, rlob, rhib, rpb, gb);
-    p2c_rev(lp, g.gLL, lcb, lpb, gb.gLL);
-    p2c_rev(rp, g.gLL, rcb, rpb, gb.gLL);
-    PrimBar lqb = zero_prim_bar(), rqb = zero_prim_bar();
-    floors_rev(o, lq, g.gLL, lpb, lqb, gb.gLL);
-    floors_rev(o, rq, g.gLL, rpb, rqb, gb.gLL);
-    qlbar[0] = lqb.rho;
-    qlbar[1] = lqb.p;
-    qrbar[0] = rqb.rho;
-    qrbar[1] = rqb.p;
-    for (int i = 0; i < 3; ++i)
+    for (int c = 0; c < 5; ++c)
+        qrbar[c] = 0.0;
+    // One side after the other: side by side their reverses do not fit the
+    // registers.  The floored primitives and conserved variables are formed
+    // again.
+    struct
     {
-        qlbar[2 + i] = lqb.v[i];
-        qrbar[2 + i] = rqb.v[i];
+        Prim q;
+        ConsBar fb, cb;
+        double lob, hib;
+    } side = {lq, lfb, lcb, llob, lhib}, next = {rq, rfb, rcb, rlob, rhib};
+#pragma unroll 1
+    for (int m = 0; m < 2; ++m)
+    {
+        Prim pf = side.q;
+        floors(o, pf, g.gLL);
+        const Cons c = p2c(pf, g.gLL);
+        PrimBar pb = zero_prim_bar(), qb = zero_prim_bar();
+        phys_flux_rev(pf, c, d, g.lapse, g.shift, side.fb, pb, side.cb,
+                      gb.lapse, gb.shift);
+        char_speeds_rev(o, pf, g, d, side.lob, side.hib, pb, gb);
+        p2c_rev(pf, g.gLL, side.cb, pb, gb.gLL);
+        floors_rev(o, side.q, g.gLL, pb, qb, gb.gLL);
+        // the left side's adjoints move over when the right one's follow
+        qlbar[0] = m ? qrbar[0] : 0.0;
+        qlbar[1] = m ? qrbar[1] : 0.0;
+        qrbar[0] = qb.rho;
+        qrbar[1] = qb.p;
+        for (int i = 0; i < 3; ++i)
+        {
+            qlbar[2 + i] = m ? qrbar[2 + i] : 0.0;
+            qrbar[2 + i] = qb.v[i];
+        }
+        side = next;
     }
     return FD;
 }

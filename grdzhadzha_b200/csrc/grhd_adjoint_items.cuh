@@ -45,10 +45,23 @@ struct AdjStage
 
 __host__ __device__ inline void cell_of(const BoxDev &b, int64_t g, int c[3])
 {
-    c[0] = b.glo[0] + (int)(g % b.gn[0]);
-    const int64_t r = g / b.gn[0];
-    c[1] = b.glo[1] + (int)(r % b.gn[1]);
-    c[2] = b.glo[2] + (int)(r / b.gn[1]);
+    // (32-bit division: a box of 2^32 cells would not fit the device)
+    const unsigned u = (unsigned)g, nx = b.gn[0], ny = b.gn[1];
+    const unsigned r = u / nx, q = r / ny;
+    c[0] = b.glo[0] + (int)(u - r * nx);
+    c[1] = b.glo[1] + (int)(r - q * ny);
+    c[2] = b.glo[2] + (int)q;
+}
+
+// Interior cell t of the box, or of one widened to n cells a side.
+__host__ __device__ inline void interior_of(const BoxDev &b, int64_t t,
+                                            const int n[3], int c[3])
+{
+    const unsigned u = (unsigned)t, nx = n[0], ny = n[1];
+    const unsigned r = u / nx, q = r / ny;
+    c[0] = b.lo[0] + (int)(u - r * nx);
+    c[1] = b.lo[1] + (int)(r - q * ny);
+    c[2] = b.lo[2] + (int)q;
 }
 
 __host__ __device__ inline int64_t stride_of(const BoxDev &b, int d)
@@ -129,10 +142,9 @@ __host__ __device__ inline void stage_tape_item(
     const double *kv, double *acc, int stage, double dt, double *out,
     double *Y, double *pY, unsigned char *br, int64_t t)
 {
-    const int i = b.lo[0] + (int)(t % b.in[0]);
-    const int64_t r = t / b.in[0];
-    const int j = b.lo[1] + (int)(r % b.in[1]);
-    const int k = b.lo[2] + (int)(r / b.in[1]);
+    int ic[3];
+    interior_of(b, t, b.in, ic);
+    const int i = ic[0], j = ic[1], k = ic[2];
     const int64_t g = b.gidx(i, j, k);
     const int comp_of[5] = {kD, kS1, kS1 + 1, kS1 + 2, kTau};
     if (excised(o, i, j, k))
@@ -173,15 +185,15 @@ __host__ __device__ inline void stage_tape_item(
     c.tau = u[4];
     double x, y, z;
     cell_xyz(o, i, j, k, x, y, z);
-    Geo geo;
-    ks_metric<double, false>(M, a, x, y, z, geo, nullptr);
+    KsCell kc;
+    ks_cell(M, a, x, y, z, kc);
     Prim pr, stored;
-    const bool ok = con2prim(o, c, geo.gUU, pr, nullptr, nullptr);
+    const bool ok = ks_con2prim(o, kc, c, pr);
     unsigned char branch;
     if (ok)
     {
         stored = pr;
-        floors(o, stored, geo.gLL);
+        ks_floors(o, kc, stored);
         branch = differs(pr, stored) ? 1 : 0;
         pY[t] = pr.p;
     }
@@ -193,7 +205,11 @@ __host__ __device__ inline void stage_tape_item(
     }
     br[t] = branch;
     if (branch)
-        c = p2c(stored, geo.gLL);
+    {
+        double gLL[6];
+        ks_gLL(kc, gLL);
+        c = p2c(stored, gLL);
+    }
     out[kRho * b.cs + g] = stored.rho;
     out[kEps * b.cs + g] = stored.eps;
     out[kPress * b.cs + g] = stored.p;
@@ -211,7 +227,7 @@ __host__ __device__ inline void stage_tape_item(
 // Face between L (index t in the direction-d face enumeration) and
 // R = L + e_d: writes the adjoints of its two reconstructed states into
 // fb[d] at L's ghosted index; returns the face's spin adjoint.
-__host__ __device__ inline double face_rev_item(const AdjRhs &A, int d,
+__host__ __device__ __forceinline__ double face_rev_item(const AdjRhs &A, int d,
                                                 int64_t t)
 {
     const BoxDev &b = A.b;
@@ -219,10 +235,7 @@ __host__ __device__ inline double face_rev_item(const AdjRhs &A, int d,
     int n[3] = {b.in[0], b.in[1], b.in[2]};
     n[d] += 1;
     int L[3];
-    L[0] = b.lo[0] + (int)(t % n[0]);
-    const int64_t r = t / n[0];
-    L[1] = b.lo[1] + (int)(r % n[1]);
-    L[2] = b.lo[2] + (int)(r / n[1]);
+    interior_of(b, t, n, L);
     L[d] -= 1;
     int R[3] = {L[0], L[1], L[2]};
     R[d] += 1;
@@ -276,17 +289,19 @@ __host__ __device__ inline double face_rev_item(const AdjRhs &A, int d,
     double xl, yl, zl, xr, yr, zr;
     cell_xyz(o, L[0], L[1], L[2], xl, yl, zl);
     cell_xyz(o, R[0], R[1], R[2], xr, yr, zr);
-    GeoT<Dual> gl, gr, gf;
-    ks_metric_spin<false>(A.M, A.a, xl, yl, zl, gl, nullptr);
-    ks_metric_spin<false>(A.M, A.a, xr, yr, zr, gr, nullptr);
-    average_geo(gl, gr, gf);
     Geo g;
-    values_of(gf, g);
-    Dual sdet(0.0);
+    {
+        Geo gl, gr;
+        ks_geo(A.M, A.a, xl, yl, zl, gl);
+        ks_geo(A.M, A.a, xr, yr, zr, gr);
+        average_geo(gl, gr, g);
+    }
     if (wacc != 0.0)
     {
-        sdet = sqrt_det(gf.gLL);
-        Fb.D += wacc * sdet.v;
+        Dual gd[6];
+        for (int q = 0; q < 6; ++q)
+            gd[q] = Dual(g.gLL[q]);
+        Fb.D += wacc * sqrt_det(gd).v;
     }
     double LL[5], Lq[5], Rq[5], RR[5];
     load5(A.P, b.pcs, gL - sd, LL);
@@ -305,9 +320,26 @@ __host__ __device__ inline double face_rev_item(const AdjRhs &A, int d,
         qlb_out[(int64_t)c * gv] = qlb[c];
         qlb_out[(int64_t)(5 + c) * gv] = qrb[c];
     }
-    double spin = contract(gb, gf);
+    // the metric's spin derivative of the two cells, one after the other and
+    // only now: held across the reverse above it would spill
+    double spin = 0.0;
+    Dual gd[6];
+    for (int q = 0; q < 6; ++q)
+        gd[q] = Dual(g.gLL[q]);
+#pragma unroll 1
+    for (int side = 0; side < 2; ++side)
+    {
+        GeoT<Dual> gs;
+        KsCellT<Dual> kd;
+        ks_cell(A.M, Dual(A.a, 1.0), side ? xr : xl, side ? yr : yl,
+                side ? zr : zl, kd);
+        ks_geo_of(kd, gs);
+        spin += 0.5 * contract(gb, gs);
+        for (int q = 0; q < 6; ++q)
+            gd[q].d += 0.5 * gs.gLL[q].d;
+    }
     if (wacc != 0.0)
-        spin += wacc * FD * sdet.d;
+        spin += wacc * FD * sqrt_det(gd).d;
     return spin;
 }
 
@@ -434,18 +466,18 @@ __host__ __device__ inline double cell_rev_item(const AdjRhs &A,
     const Options &o = A.o;
     const int64_t gv = b.gvol();
     int c[3];
-    c[0] = b.lo[0] + (int)(t % b.in[0]);
-    const int64_t r = t / b.in[0];
-    c[1] = b.lo[1] + (int)(r % b.in[1]);
-    c[2] = b.lo[2] + (int)(r / b.in[1]);
+    interior_of(b, t, b.in, c);
     const int64_t g = b.gidx(c[0], c[1], c[2]);
     const int64_t rcs = b.rcs;
     ConsBar Ub = zero_cons_bar();
     double spin = 0.0;
     const bool exc = excised(o, c[0], c[1], c[2]);
-    GeoFullT<Dual> fd;
-    GeoFullBar fbar;
-    zero(fbar);
+    double x, y, z;
+    cell_xyz(o, c[0], c[1], c[2], x, y, z);
+    KsCellT<Dual> kd; // the cell and its spin derivative
+    Geo ge;
+    GeoBar gb;
+    zero(gb);
     if (!exc)
     {
         double lp[5] = {0, 0, 0, 0, 0};
@@ -469,11 +501,12 @@ __host__ __device__ inline double cell_rev_item(const AdjRhs &A,
         cb.p = lp[1];
         for (int i = 0; i < 3; ++i)
             cb.v[i] = lp[2 + i];
-        double x, y, z;
-        cell_xyz(o, c[0], c[1], c[2], x, y, z);
-        ks_metric_spin<true>(A.M, A.a, x, y, z, fd.g, &fd);
-        GeoFull f;
-        values_of(fd, f);
+        ks_cell(A.M, Dual(A.a, 1.0), x, y, z, kd);
+        {
+            GeoT<Dual> gd;
+            ks_geo_of(kd, gd);
+            values_of(gd, ge);
+        }
         const Cons U = load_cons5(A.U, b.cs, g);
         double q5[5];
         load5(A.P, b.pcs, g, q5);
@@ -486,16 +519,30 @@ __host__ __device__ inline double cell_rev_item(const AdjRhs &A,
         if (o.use_src)
         {
             Prim fl = pr;
-            floors(o, fl, f.g.gLL);
+            floors(o, fl, ge.gLL);
             if (!is_atmo(o, fl, o.src_atmo_factor))
             {
                 const ConsBar sb = lamk_at(A, t);
                 PrimBar flb = zero_prim_bar();
-                static_sources_rev(fl, U, f, sb, flb, Ub, fbar);
-                floors_rev(o, pr, f.g.gLL, flb, cb, fbar.g.gLL);
+                {
+                    // the metric's adjoint is not formed (it and the
+                    // metric are 55 numbers each): the spin derivative of
+                    // the sources comes from their own dual numbers
+                    GeoFull f;
+                    GeoFullBar unused;
+                    zero(unused);
+                    ks_metric<double, true>(A.M, A.a, x, y, z, f.g, &f);
+                    static_sources_rev(fl, U, f, sb, flb, Ub, unused);
+                }
+                fl.eps = fl.p * rcp_ulp((o.G - 1.0) * fl.rho);
+                const ConsT<Dual> s = ks_sources(o, Dual(A.a, 1.0), kd, x, y,
+                                                 z, fl, U);
+                spin += sb.D * s.D.d + sb.tau * s.tau.d + sb.S[0] * s.S[0].d +
+                        sb.S[1] * s.S[1].d + sb.S[2] * s.S[2].d;
+                floors_rev(o, pr, ge.gLL, flb, cb, gb.gLL);
             }
         }
-        con2prim_rev(o, U, f.g.gUU, pr.p, cb, Ub, fbar.g.gUU);
+        con2prim_rev(o, U, ge.gUU, pr.p, cb, Ub, gb.gUU);
     }
     // stage combination and recovery
     if (S.stage >= 1)
@@ -509,9 +556,7 @@ __host__ __device__ inline double cell_rev_item(const AdjRhs &A,
             Y.S[1] = S.Y[2 * rcs + t];
             Y.S[2] = S.Y[3 * rcs + t];
             Y.tau = S.Y[4 * rcs + t];
-            Geo g2;
-            values_of(fd.g, g2);
-            B = recovery_rev(o, Y, S.br[t], S.pY[t], g2, Ub, fbar.g);
+            B = recovery_rev(o, Y, S.br[t], S.pY[t], ge, Ub, gb);
         }
         const double Bv[5] = {B.D, B.S[0], B.S[1], B.S[2], B.tau};
         // lambda_k of the previous stage: cA A + cB B
@@ -532,7 +577,11 @@ __host__ __device__ inline double cell_rev_item(const AdjRhs &A,
                 (S.stage == 0 ? S.acc[q * rcs + t] : 0.0) + Uv[q];
     }
     if (!exc)
-        spin += contract(fbar, fd);
+    {
+        GeoT<Dual> gd;
+        ks_geo_of(kd, gd);
+        spin += contract(gb, gd);
+    }
     return spin;
 }
 
@@ -544,10 +593,9 @@ __host__ __device__ inline double proj_rev_item(
     const unsigned char *br, double *A, double *acc, double *lamk, int64_t t)
 {
     const int64_t rcs = b.rcs;
-    const int i = b.lo[0] + (int)(t % b.in[0]);
-    const int64_t r = t / b.in[0];
-    const int j = b.lo[1] + (int)(r % b.in[1]);
-    const int k = b.lo[2] + (int)(r / b.in[1]);
+    int ic[3];
+    interior_of(b, t, b.in, ic);
+    const int i = ic[0], j = ic[1], k = ic[2];
     ConsBar Ub;
     Ub.D = lam[0 * rcs + t];
     Ub.S[0] = lam[1 * rcs + t];
@@ -633,10 +681,9 @@ __host__ __device__ inline void torus_tangent_item(const TorusArgs &T,
                                                    double acc[8])
 {
     const BoxDev &b = T.b;
-    const int i = b.lo[0] + (int)(t % b.in[0]);
-    const int64_t r = t / b.in[0];
-    const int j = b.lo[1] + (int)(r % b.in[1]);
-    const int k = b.lo[2] + (int)(r / b.in[1]);
+    int ic[3];
+    interior_of(b, t, b.in, ic);
+    const int i = ic[0], j = ic[1], k = ic[2];
     double x, y, z;
     cell_xyz(T.o, i, j, k, x, y, z);
     for (int p = 0; p < 8; ++p)

@@ -379,44 +379,48 @@ GRHD_HD __forceinline__ void ks_metric(T M, T a, T x, T y, T z,
 
 // An FP64 Kerr-Schild cell in terms of its null vector l and H (see "FP64
 // Kerr-Schild cell" below).
-struct KsCell
+// T = double, or the dual numbers of the adjoint's spin derivative.
+template <typename T> struct KsCellT
 {
-    double l[3], F, c, alpha, alpha2;
-    double r, inv_r, inv_ra, inv_sigma; // 1/r, 1/(r^2 + a^2), 1/Sigma
+    T l[3], F, c, alpha, alpha2;
+    T r, inv_r, inv_ra, inv_sigma; // 1/r, 1/(r^2 + a^2), 1/Sigma
 };
+using KsCell = KsCellT<double>;
 
-GRHD_HD __forceinline__ void ks_cell(double M, double a, double x, double y,
-                                     double z, KsCell &k)
+template <typename T>
+GRHD_HD __forceinline__ void ks_cell(double M, T a, double x, double y,
+                                     double z, KsCellT<T> &k)
 {
-    const double a2 = mul_(a, a);
+    const T a2 = mul_(a, a);
     const double rho2 =
         fmax(fma(x, x, fma(y, y, mul_(z, z))), 1.0e-12); // (1e-6)^2
-    const double hA = 0.5 * (rho2 - a2);
-    const double az = mul_(a, z);
-    const double r2 = hA + sqrt_(fma(hA, hA, mul_(az, az)));
+    const T hA = 0.5 * (rho2 - a2);
+    const T az = mul_(a, z);
+    const T r2 = hA + sqrt_(fma(hA, hA, mul_(az, az)));
     // r and 1/r from one reciprocal square root, each corrected once
-    const double y0 = rsqrt_ulp(r2);
-    const double r0 = mul_(r2, y0);
-    const double r = fma(fma(-r0, r0, r2), 0.5 * y0, r0);
+    const T y0 = rsqrt_ulp(r2);
+    const T r0 = mul_(r2, y0);
+    const T r = fma(fma(-r0, r0, r2), 0.5 * y0, r0);
     k.r = r;
     k.inv_r = fma(fma(-r, y0, 1.0), y0, y0);
-    const double ct = mul_(z, k.inv_r);
-    const double act = mul_(a, ct);
+    const T ct = mul_(z, k.inv_r);
+    const T act = mul_(a, ct);
     k.inv_sigma = rcp_ulp(fma(act, act, r2));
     k.inv_ra = rcp_ulp(r2 + a2);
     k.l[0] = mul_(fma(r, x, mul_(a, y)), k.inv_ra);
     k.l[1] = mul_(fma(r, y, -mul_(a, x)), k.inv_ra);
     k.l[2] = ct;
     k.F = mul_(mul_(2.0 * M, r), k.inv_sigma);
-    const double u = 1.0 + k.F;
+    const T u = 1.0 + k.F;
     k.alpha2 = rcp_ulp(u);
     k.alpha = rsqrt_ulp(u);
     k.c = mul_(k.F, k.alpha2);
 }
 
-GRHD_HD __forceinline__ void ks_gLL(const KsCell &k, double g[6])
+template <typename T>
+GRHD_HD __forceinline__ void ks_gLL(const KsCellT<T> &k, T g[6])
 {
-    const double f[3] = {mul_(k.F, k.l[0]), mul_(k.F, k.l[1]),
+    const T f[3] = {mul_(k.F, k.l[0]), mul_(k.F, k.l[1]),
                          mul_(k.F, k.l[2])};
     g[0] = fma(f[0], k.l[0], 1.0);
     g[1] = mul_(f[0], k.l[1]);
@@ -428,11 +432,9 @@ GRHD_HD __forceinline__ void ks_gLL(const KsCell &k, double g[6])
 
 // The face geometry of a cell from them: 60 FP64 operations and five special
 // functions against some 90 and eight of ks_metric's general sequence.
-GRHD_HD __forceinline__ void ks_geo(double M, double a, double x, double y,
-                                    double z, Geo &g)
+template <typename T>
+GRHD_HD __forceinline__ void ks_geo_of(const KsCellT<T> &k, GeoT<T> &g)
 {
-    KsCell k;
-    ks_cell(M, a, x, y, z, k);
     ks_gLL(k, g.gLL);
 #pragma unroll
     for (int i = 0; i < 3; ++i)
@@ -442,8 +444,16 @@ GRHD_HD __forceinline__ void ks_geo(double M, double a, double x, double y,
 #pragma unroll
         for (int j = i; j < 3; ++j)
             g.gUU[sym(i, j)] =
-                fma(-g.shift[i], k.l[j], i == j ? 1.0 : 0.0);
+                fma(-g.shift[i], k.l[j], T(i == j ? 1.0 : 0.0));
     g.lapse = k.alpha;
+}
+
+GRHD_HD __forceinline__ void ks_geo(double M, double a, double x, double y,
+                                    double z, Geo &g)
+{
+    KsCell k;
+    ks_cell(M, a, x, y, z, k);
+    ks_geo_of(k, g);
 }
 
 // Softened circular-binary potentials at `pos` (add_point_potential,
@@ -818,7 +828,8 @@ GRHD_HD __forceinline__ void raise(const double gUU[6], const double S[3],
     mU[2] = fma(gUU[2], S[0], fma(gUU[4], S[1], mul_(gUU[5], S[2])));
 }
 
-GRHD_HD __forceinline__ double dot3(const double a[3], const double b[3])
+template <typename A, typename B>
+GRHD_HD __forceinline__ auto dot3(const A a[3], const B b[3])
 {
     return fma(a[0], b[0], fma(a[1], b[1], mul_(a[2], b[2])));
 }
@@ -1527,10 +1538,11 @@ GRHD_HD __forceinline__ ConsT<T> static_sources(const PrimT<T> &pr,
 // spill: 2.77 -> 1.55 ms per launch at 256^3 (bytes alone: 0.72), the RK4
 // step 21.0 -> 15.8 ms.
 // gamma^ij S_j
-GRHD_HD __forceinline__ void ks_raise(const KsCell &k, const double S[3],
-                                      double mU[3])
+template <typename T>
+GRHD_HD __forceinline__ void ks_raise(const KsCellT<T> &k, const double S[3],
+                                      T mU[3])
 {
-    const double t = mul_(k.c, dot3(k.l, S));
+    const T t = mul_(k.c, dot3(k.l, S));
     mU[0] = fma(-t, k.l[0], S[0]);
     mU[1] = fma(-t, k.l[1], S[1]);
     mU[2] = fma(-t, k.l[2], S[2]);
@@ -1581,82 +1593,84 @@ GRHD_HD __forceinline__ bool ks_con2prim(const Options &o, const KsCell &k,
 //             delta_iy) / (r^2 + a^2) + u_z delta_iz / r,
 //   w(u) = (u_x (x - 2 r l_x) + u_y (y - 2 r l_y)) / (r^2 + a^2)
 //          - u_z l_z / r.
-GRHD_HD __forceinline__ Cons ks_sources(const Options &o, double a,
-                                        const KsCell &k, double x, double y,
-                                        double z, const Prim &pr,
-                                        const Cons &c)
+template <typename T>
+GRHD_HD __forceinline__ ConsT<T> ks_sources(const Options &o, T a,
+                                            const KsCellT<T> &k, double x,
+                                            double y, double z,
+                                            const Prim &pr, const Cons &c)
 {
-    const double a2 = mul_(a, a);
-    const double *l = k.l, *v = pr.v;
+    const T a2 = mul_(a, a);
+    const T *l = k.l;
+    const double *v = pr.v;
     // d r, d H
-    const double rs = mul_(k.r, k.inv_sigma);
-    const double ias = mul_(k.inv_r, k.inv_sigma);
-    const double dr[3] = {mul_(rs, x), mul_(rs, y),
+    const T rs = mul_(k.r, k.inv_sigma);
+    const T ias = mul_(k.inv_r, k.inv_sigma);
+    const T dr[3] = {mul_(rs, x), mul_(rs, y),
                           mul_(fma(a2, ias, rs), z)};
-    const double H = 0.5 * k.F;
-    const double a2ct = mul_(a2, l[2]);
+    const T H = 0.5 * k.F;
+    const T a2ct = mul_(a2, l[2]);
     // r - a^2 ct^2 / r
-    const double rm = fma(-mul_(a2ct, l[2]), k.inv_r, k.r);
-    const double hk = mul_(H, fma(mul_(-2.0, k.inv_sigma), rm, k.inv_r));
-    const double dH[3] = {mul_(hk, dr[0]), mul_(hk, dr[1]),
+    const T rm = fma(-mul_(a2ct, l[2]), k.inv_r, k.r);
+    const T hk = mul_(H, fma(mul_(-2.0, k.inv_sigma), rm, k.inv_r));
+    const T dH[3] = {mul_(hk, dr[0]), mul_(hk, dr[1]),
                           fma(hk, dr[2], -mul_(mul_(k.F, a2ct), ias))};
-    const double vH = dot3(v, dH), lH = dot3(l, dH);
-    double mU[3];
+    const T vH = dot3(v, dH), lH = dot3(l, dH);
+    T mU[3];
     ks_raise(k, c.S, mU);
-    const double mH = dot3(mU, dH), Sl = dot3(c.S, l);
+    const T mH = dot3(mU, dH), Sl = dot3(c.S, l);
     // rho h W^2, v.l
-    const double lv = dot3(l, v);
-    const double vv = fma(mul_(k.F, lv), lv, dot3(v, v));
-    const double rhw = mul_(mul_(pr.rho, fma(o.G, pr.eps, 1.0)),
+    const T lv = dot3(l, v);
+    const T vv = fma(mul_(k.F, lv), lv, dot3(v, v));
+    const T rhw = mul_(mul_(pr.rho, fma(o.G, pr.eps, 1.0)),
                             rcp_ulp(1.0 - vv));
-    const double rl = mul_(rhw, lv);
+    const T rl = mul_(rhw, lv);
     // l_i T^ij l_j of the stress T^ij = rhw v^i v^j + p gamma^ij
-    const double lTl = fma(rl, lv, mul_(pr.p, k.alpha2));
+    const T lTl = fma(rl, lv, mul_(pr.p, k.alpha2));
     // transport velocity along d ln sqrt(gamma)
-    const double T =
+    const T tv =
         mul_(k.alpha2, fma(k.alpha, vH, -mul_(k.c, lH)));
     // w(u), v.dl.v and div l
-    const double tr = 2.0 * k.r;
-    const double wx = mul_(fma(-tr, l[0], x), k.inv_ra);
-    const double wy = mul_(fma(-tr, l[1], y), k.inv_ra);
-    const double wz = -mul_(l[2], k.inv_r);
-    const double ri = mul_(k.r, k.inv_ra);
-    const double wv = fma(v[0], wx, fma(v[1], wy, mul_(v[2], wz)));
-    const double vA =
+    const T tr = 2.0 * k.r;
+    const T wx = mul_(fma(-tr, l[0], x), k.inv_ra);
+    const T wy = mul_(fma(-tr, l[1], y), k.inv_ra);
+    const T wz = -mul_(l[2], k.inv_r);
+    const T ri = mul_(k.r, k.inv_ra);
+    const T wv = fma(v[0], wx, fma(v[1], wy, mul_(v[2], wz)));
+    const T vA =
         fma(dot3(v, dr), wv,
             fma(ri, fma(v[0], v[0], mul_(v[1], v[1])),
                 mul_(mul_(v[2], v[2]), k.inv_r)));
-    const double div = fma(dr[0], wx, fma(dr[1], wy, fma(dr[2], wz,
+    const T div = fma(dr[0], wx, fma(dr[1], wy, fma(dr[2], wz,
                            fma(2.0, ri, k.inv_r))));
-    Cons s;
-    s.D = -mul_(c.D, T);
-    const double aa2 = mul_(k.alpha, k.alpha2);
+    ConsT<T> s;
+    s.D = -mul_(c.D, tv);
+    const T aa2 = mul_(k.alpha, k.alpha2);
     // alpha T^ij K_ij
-    const double db = 2.0 * k.alpha2; // d_i beta^j = db alpha^2 D_i l^j + ...
-    const double TK =
+    const T db = 2.0 * k.alpha2; // d_i beta^j = db alpha^2 D_i l^j + ...
+    const T TK =
         fma(mul_(lTl, k.c), lH,
             fma(rl, mul_(db, vH),
                 fma(mul_(rhw, k.c), vA,
                     mul_(pr.p, fma(mul_(db, k.alpha2), lH,
                                    mul_(k.c, div))))));
-    s.tau = fma(aa2, fma(-pr.p, vH, mH), fma(-c.tau, T, TK));
+    s.tau = fma(aa2, fma(-pr.p, vH, mH), fma(-c.tau, tv, TK));
     // momentum: u.d_m l with u = alpha F rhw (v.l) v + c S
-    const double X =
-        fma(aa2, (c.D + c.tau) - pr.p,
+    const T X =
+        fma(aa2, T((c.D + c.tau) - pr.p),
             fma(k.alpha, lTl, mul_(mul_(db, k.alpha2), Sl)));
-    const double q = mul_(mul_(k.alpha, k.F), rl);
-    const double u[3] = {fma(q, v[0], mul_(k.c, c.S[0])),
+    const T q = mul_(mul_(k.alpha, k.F), rl);
+    const T u[3] = {fma(q, v[0], mul_(k.c, c.S[0])),
                          fma(q, v[1], mul_(k.c, c.S[1])),
                          fma(q, v[2], mul_(k.c, c.S[2]))};
-    const double wu = fma(u[0], wx, fma(u[1], wy, mul_(u[2], wz)));
-    const double ai = mul_(a, k.inv_ra);
-    const double g[3] = {fma(ri, u[0], -mul_(ai, u[1])),
+    const T wu = fma(u[0], wx, fma(u[1], wy, mul_(u[2], wz)));
+    const T ai = mul_(a, k.inv_ra);
+    const T g[3] = {fma(ri, u[0], -mul_(ai, u[1])),
                          fma(ri, u[1], mul_(ai, u[0])),
                          mul_(u[2], k.inv_r)};
 #pragma unroll
     for (int m = 0; m < 3; ++m)
         s.S[m] = fma(dH[m], X,
-                     fma(dr[m], wu, fma(-c.S[m], T, g[m])));
+                     fma(dr[m], wu, fma(-c.S[m], tv, g[m])));
     return s;
 }
 

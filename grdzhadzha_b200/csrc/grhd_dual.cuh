@@ -2,7 +2,8 @@
 // derivative) for the spin derivative of the analytic metric and of the
 // torus initial data.  The metric and torus functions are templates on
 // their arithmetic type; instantiated with Dual and the spin seeded with
-// derivative 1 they return each quantity together with d/da.
+// derivative 1 they return each quantity together with d/da.  Quotients and
+// roots share one one-ulp reciprocal between value and derivative.
 #pragma once
 
 #include "grhd_device.cuh"
@@ -28,8 +29,9 @@ GRHD_HD inline Dual operator*(Dual a, Dual b)
 }
 GRHD_HD inline Dual operator/(Dual a, Dual b)
 {
-    const double q = a.v / b.v;
-    return Dual(q, (a.d - q * b.d) / b.v);
+    const double r = rcp_ulp(b.v);
+    const double q = a.v * r;
+    return Dual(q, (a.d - q * b.d) * r);
 }
 GRHD_HD inline Dual operator+(Dual a, double b) { return Dual(a.v + b, a.d); }
 GRHD_HD inline Dual operator+(double a, Dual b) { return Dual(a + b.v, b.d); }
@@ -37,11 +39,16 @@ GRHD_HD inline Dual operator-(Dual a, double b) { return Dual(a.v - b, a.d); }
 GRHD_HD inline Dual operator-(double a, Dual b) { return Dual(a - b.v, -b.d); }
 GRHD_HD inline Dual operator*(Dual a, double b) { return Dual(a.v * b, a.d * b); }
 GRHD_HD inline Dual operator*(double a, Dual b) { return Dual(a * b.v, a * b.d); }
-GRHD_HD inline Dual operator/(Dual a, double b) { return Dual(a.v / b, a.d / b); }
+GRHD_HD inline Dual operator/(Dual a, double b) 
+{
+    const double r = rcp_ulp(b);
+    return Dual(a.v * r, a.d * r);
+}
 GRHD_HD inline Dual operator/(double a, Dual b)
 {
-    const double q = a / b.v;
-    return Dual(q, -q * b.d / b.v);
+    const double r = rcp_ulp(b.v);
+    const double q = a * r;
+    return Dual(q, -q * b.d * r);
 }
 GRHD_HD inline Dual &operator+=(Dual &a, Dual b)
 {
@@ -67,15 +74,27 @@ GRHD_HD inline Dual div_(Dual a, Dual b) { return a / b; }
 GRHD_HD inline Dual rcp_(Dual a) { return 1.0 / a; }
 GRHD_HD inline Dual sqrt_(Dual a)
 {
-    const double s = sqrt(a.v);
-    return Dual(s, a.d / (2.0 * s));
+    const double s = sqrt_(a.v);
+    return Dual(s, 0.5 * a.d * rcp_ulp(s));
 }
 GRHD_HD inline Dual rsqrt_(Dual a)
 {
-    const double r = 1.0 / sqrt(a.v);
+    const double r = rsqrt_ulp(a.v);
     return Dual(r, -0.5 * r * r * r * a.d);
 }
 GRHD_HD inline Dual lapse_rsqrt(Dual a) { return rsqrt_(a); }
+// The names the Kerr-Schild cell is written in (grhd_device.cuh).
+GRHD_HD inline Dual mul_(Dual a, Dual b) { return a * b; }
+GRHD_HD inline Dual fma(Dual a, Dual b, Dual c)
+{
+    return Dual(::fma(a.v, b.v, c.v), ::fma(a.d, b.v, ::fma(a.v, b.d, c.d)));
+}
+GRHD_HD inline Dual rcp_ulp(Dual a)
+{
+    const double r = rcp_ulp(a.v);
+    return Dual(r, -r * r * a.d);
+}
+GRHD_HD inline Dual rsqrt_ulp(Dual a) { return rsqrt_(a); }
 // max/min return the selected operand (derivative included)
 GRHD_HD inline Dual max_(Dual a, Dual b) { return (a.v >= b.v) ? a : b; }
 GRHD_HD inline Dual min_(Dual a, Dual b) { return (a.v <= b.v) ? a : b; }
