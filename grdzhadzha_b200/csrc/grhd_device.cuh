@@ -492,7 +492,8 @@ __device__ __forceinline__ void pn_add_point(T mass, T soft2, const double *sp,
 // with step h (FixedBGFArrayBoxFiniteVolume.hpp:616-631), which amplifies
 // the rounding of U by ~1/h; the sums here are written with
 // round-to-nearest intrinsics so that no multiply-add is fused and U rounds
-// exactly as the reference's expression does.
+// as the reference's expression does (sqrt_ and rcp_ give the IEEE results on
+// every tested operand, without the IEEE operations' slow-path branches).
 __device__ __forceinline__ double pn_scalar(double m1, double m2,
                                             double soft2, const double *p1,
                                             const double *p2,
@@ -507,8 +508,8 @@ __device__ __forceinline__ double pn_scalar(double m1, double m2,
         r1 = __dadd_rn(r1, __dmul_rn(d1, d1));
         r2 = __dadd_rn(r2, __dmul_rn(d2, d2));
     }
-    return __dadd_rn(__dmul_rn(m1, 1.0 / sqrt(r1)),
-                     __dmul_rn(m2, 1.0 / sqrt(r2)));
+    return __dadd_rn(__dmul_rn(m1, rcp_(sqrt_(r1))),
+                     __dmul_rn(m2, rcp_(sqrt_(r2))));
 }
 
 // CircularBinaryPN::compute_metric_background, CircularBinaryPN.hpp:70-189:

@@ -402,9 +402,9 @@ __device__ __forceinline__ ConsT<T> cell_sources(const Options &o,
         const double Up = pn_scalar(bg.m1, bg.m2, bg.soft2, bg.p1p, bg.p2p, pos);
         const double Um = pn_scalar(bg.m1, bg.m2, bg.soft2, bg.p1m, bg.p2m, pos);
         const double dl =
-            __dadd_rn(pn_log_sqrt_det(__dadd_rn(1.0, 2.0 * Up)),
-                      -pn_log_sqrt_det(__dadd_rn(1.0, 2.0 * Um))) /
-            (2.0 * bg.fd_h);
+            div_(__dadd_rn(pn_log_sqrt_det(__dadd_rn(1.0, 2.0 * Up)),
+                           -pn_log_sqrt_det(__dadd_rn(1.0, 2.0 * Um))),
+                 2.0 * bg.fd_h);
         s.D = T(double(s.D) + (0.0 - c.D * dl));
         s.tau = T(double(s.tau) + (0.0 - c.tau * dl));
 #pragma unroll
@@ -2875,7 +2875,7 @@ void launch_cells(const double *state, T *prim, T *src, const BoxDev &b,
         kern<<<grid_for(b.ivol(), 256), 256, 0, s>>>(state, prim, src, b, bg,
                                                      o, st);
     };
-    if (sizeof(T) == sizeof(float))
+    if constexpr (sizeof(T) == sizeof(float))
         go(k_cells<T, -1>);
     else
         bg.kind == 1 ? go(k_cells<T, 1>) : go(k_cells<T, 0>);
