@@ -673,8 +673,7 @@ int grhd_recover_primitives(grhd_ctx *ctx, double *state, int64_t state_cs,
     const Background bg = make_background(ctx->params, time);
     {
         Timed t_(ctx, GRHD_K_STAGE, s);
-        launch_recover(state, b, bg, ctx->opt, ctx->status,
-                       ctx->params.precision == GRHD_PRECISION_MIXED, s);
+        launch_recover(state, b, bg, ctx->opt, ctx->status, s);
     }
     st = finish_status(ctx, b, state, bg, s);
     read_diag(ctx, diag);
@@ -703,8 +702,7 @@ int grhd_update_conserved(grhd_ctx *ctx, double *state, int64_t state_cs,
     {
         Timed t_(ctx, GRHD_K_STAGE, s);
         launch_update(state, b.cs, state, b.cs, rhs, b, bg, ctx->opt, dt,
-                      recover, ctx->status,
-                      ctx->params.precision == GRHD_PRECISION_MIXED, s);
+                      recover, ctx->status, s);
     }
     st = finish_status(ctx, b, state, bg, s);
     read_diag(ctx, diag);

@@ -1173,20 +1173,6 @@ GRHD_HD __forceinline__ void char_speeds(const Options &o,
     char_speeds_k(T(o.G), pr, g, d, lo, hi);
 }
 
-// minmod / compute_limited_slope, Reconstruction.hpp:16-37
-template <typename T> GRHD_HD __forceinline__ T minmod2(T l, T r)
-{
-    if (l * r <= T(0))
-        return T(0);
-    return l > T(0) ? min_(l, r) : max_(l, r);
-}
-
-template <typename T>
-GRHD_HD __forceinline__ T limited_slope(T l, T c, T r, T theta)
-{
-    return minmod2(theta * (c - l), minmod2(T(0.5) * (r - l), theta * (r - c)));
-}
-
 // The constants of a face flux in its arithmetic type, made once per launch
 // (as kernel parameters they are operands in the constant bank; the options'
 // FP64 members cost the FP32 path a conversion at each use).
@@ -1336,8 +1322,8 @@ GRHD_HD __forceinline__ double slope_of(double l, double c, double r,
 {
     return limited_slope_f64(l, c, r, theta);
 }
-// The same in FP32 (limited_slope's value bit for bit while the products of
-// two slopes do not underflow, 1e-45): 14 instructions instead of 21; the
+// The same in FP32 (the nested minmod's value bit for bit while the products
+// of two slopes do not underflow, 1e-45): 14 instructions instead of 21; the
 // mixed face kernel, issue-bound, went from 1.66 to 1.43 ms at 256^3.
 __device__ __forceinline__ float slope_of(float l, float c, float r,
                                           float theta)

@@ -1054,16 +1054,18 @@ __global__ void k_mdot_sum(const double *__restrict__ part, int64_t n,
 
 // recover_primitives_and_apply_atmosphere_from_fixed_background for one
 // cell (FixedBGFArrayBoxFiniteVolume.hpp:60-110); c is the updated
-// conserved state.  Writes prims (and reset conserved) to `out`.  T picks the
-// path's root solve (the metric is FP64 in both).
-template <typename T>
+// conserved state.  Writes prims (and reset conserved) to `out`.  With kc the
+// root solve is the Kerr-Schild cell's, the FP64 right-hand side's own: a
+// state's recovered pressures are those its right-hand side starts from.
 __device__ __forceinline__ void recover_cell(const Options &o, const Geo &g,
-                                             Cons c, double *out, int64_t cs,
+                                             const KsCell *kc, Cons c,
+                                             double *out, int64_t cs,
                                              int64_t idx,
                                              unsigned long long cnt[4])
 {
     Prim pr;
-    const bool ok = cold_con2prim<T>(o, c, g.gUU, pr);
+    const bool ok = kc ? ks_con2prim(o, *kc, c, pr)
+                       : con2prim(o, c, g.gUU, pr, nullptr, nullptr);
     bool reset = !ok;
     cnt[0] += 1;
     if (ok)
@@ -1113,7 +1115,6 @@ __device__ __forceinline__ void flush_counts(DevStatus *st,
 // update_conserved: dst = src + dt * rhs on the interior
 // (add_scaled_conserved_rhs, FArrayBoxFiniteVolume.hpp:927-940), then the
 // post-update recovery when `recover` is set.
-template <typename T>
 __global__ void __launch_bounds__(256)
     k_update(double *dst, int64_t dcs, const double *srcs, int64_t scs,
              const double *__restrict__ rhs, BoxDev b, Background bg,
@@ -1150,7 +1151,11 @@ __global__ void __launch_bounds__(256)
                     cell_xyz(o, i, j, k, x, y, z);
                     Geo geo;
                     background_metric<false>(bg, x, y, z, geo, nullptr);
-                    recover_cell<T>(o, geo, c, dst, dcs, g, cnt);
+                    KsCell kc;
+                    if (bg.kind == 0)
+                        ks_cell(bg.M, bg.a, x, y, z, kc);
+                    recover_cell(o, geo, bg.kind == 0 ? &kc : nullptr, c, dst,
+                                 dcs, g, cnt);
                 }
                 else
                 {
@@ -1165,7 +1170,6 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-template <typename T>
 __global__ void __launch_bounds__(256)
     k_recover(double *__restrict__ state, BoxDev b, Background bg, Options o,
               DevStatus *st)
@@ -1187,8 +1191,11 @@ __global__ void __launch_bounds__(256)
                 cell_xyz(o, i, j, k, x, y, z);
                 Geo geo;
                 background_metric<false>(bg, x, y, z, geo, nullptr);
-                recover_cell<T>(o, geo, load_cons(state, b.cs, g), state, b.cs,
-                                g, cnt);
+                KsCell kc;
+                if (bg.kind == 0)
+                    ks_cell(bg.M, bg.a, x, y, z, kc);
+                recover_cell(o, geo, bg.kind == 0 ? &kc : nullptr,
+                             load_cons(state, b.cs, g), state, b.cs, g, cnt);
             }
         }
         flush_counts(st, cnt);
@@ -1248,7 +1255,7 @@ __global__ void __launch_bounds__(256)
             {
                 Geo geo;
                 background_metric<false, 1>(bg, x, y, z, geo, nullptr);
-                recover_cell<double>(o, geo, c, s, b.cs, g, cnt);
+                recover_cell(o, geo, nullptr, c, s, b.cs, g, cnt);
             }
         }
         flush_counts(st, cnt);
@@ -2545,7 +2552,7 @@ __global__ void __launch_bounds__(256)
                 geo = geo_get(gc, b.gvol(), g);
             else
                 ccz4_geo(m, mcs, g, geo, nullptr);
-            recover_cell<double>(o, geo, c, out, ocs, g, cnt);
+            recover_cell(o, geo, nullptr, c, out, ocs, g, cnt);
         }
         flush_counts(st, cnt);
         cnt[0] = cnt[1] = cnt[2] = cnt[3] = 0;
@@ -2570,8 +2577,8 @@ __global__ void __launch_bounds__(256)
             const int64_t g = b.gidx(i, j, k);
             Geo geo;
             ccz4_geo(s, b.cs, g, geo, nullptr);
-            recover_cell<double>(o, geo, load_cons(q, b.cs, g), q, b.cs, g,
-                                 cnt);
+            recover_cell(o, geo, nullptr, load_cons(q, b.cs, g), q, b.cs, g,
+                         cnt);
         }
         flush_counts(st, cnt);
         cnt[0] = cnt[1] = cnt[2] = cnt[3] = 0;
@@ -2933,23 +2940,16 @@ void launch_mdot_sum(const double *part, int64_t n, double weight,
 void launch_update(double *dst, int64_t dcs, const double *src_state,
                    int64_t scs, const double *rhs, const BoxDev &b,
                    const Background &bg, const Options &o, double dt,
-                   int recover, DevStatus *st, bool mixed, cudaStream_t s)
+                   int recover, DevStatus *st, cudaStream_t s)
 {
-    auto go = [&](auto kern) {
-        kern<<<grid_for(b.ivol(), 256), 256, 0, s>>>(
-            dst, dcs, src_state, scs, rhs, b, bg, o, dt, recover, st);
-    };
-    mixed ? go(k_update<float>) : go(k_update<double>);
+    k_update<<<grid_for(b.ivol(), 256), 256, 0, s>>>(
+        dst, dcs, src_state, scs, rhs, b, bg, o, dt, recover, st);
 }
 
 void launch_recover(double *state, const BoxDev &b, const Background &bg,
-                    const Options &o, DevStatus *st, bool mixed,
-                    cudaStream_t s)
+                    const Options &o, DevStatus *st, cudaStream_t s)
 {
-    auto go = [&](auto kern) {
-        kern<<<grid_for(b.ivol(), 256), 256, 0, s>>>(state, b, bg, o, st);
-    };
-    mixed ? go(k_recover<float>) : go(k_recover<double>);
+    k_recover<<<grid_for(b.ivol(), 256), 256, 0, s>>>(state, b, bg, o, st);
 }
 
 // Blocks of a stage launch: two cells a thread where that leaves four waves

@@ -186,15 +186,13 @@ void launch_faces(const T *prim, const T *src, T *rhs, const BoxDev &b,
 // acc[0] = sum of part[0..n); acc[1] += weight * acc[0]
 void launch_mdot_sum(const double *part, int64_t n, double weight,
                      double *acc, cudaStream_t s);
-// update_conserved (FP64; `mixed` picks that path's root solve): dst = src +
-// dt rhs, then recovery when asked.
+// update_conserved (FP64): dst = src + dt rhs, then recovery when asked.
 void launch_update(double *dst, int64_t dcs, const double *src_state,
                    int64_t scs, const double *rhs, const BoxDev &b,
                    const Background &bg, const Options &o, double dt,
-                   int recover, DevStatus *st, bool mixed, cudaStream_t s);
+                   int recover, DevStatus *st, cudaStream_t s);
 void launch_recover(double *state, const BoxDev &b, const Background &bg,
-                    const Options &o, DevStatus *st, bool mixed,
-                    cudaStream_t s);
+                    const Options &o, DevStatus *st, cudaStream_t s);
 // Integrator stage fused with the post-update recovery; mode 0 RK4 stage
 // `stage`, 1 Euler update, 2 SSPRK2 combine.  With prep the stage also
 // prepares the next RHS (primitive cache and sources); the mixed path

@@ -2,7 +2,9 @@
 // cell in terms of l and H (ks_cell, ks_floors, ks_sources, ks_inverse_dt)
 // against the general metric with its derivatives (ks_metric,
 // static_sources, char_speeds), and the root solve with overlapped residuals
-// (c2p_solve) against the one that evaluates them in turn (con2prim_mixed).
+// (c2p_solve) against the one that evaluates them in turn (con2prim_mixed),
+// the limited slope against the nested minmod (equal values), and the face
+// flux with shared subexpressions against its separate formulas.
 //
 // Tolerances.  Metric, sources and speeds: some 200 roundings of 1.1e-16,
 // conditioned at r >= 2 by at most 10, of the terms' size: 1e-12.  Pressure:
@@ -130,6 +132,94 @@ void cell(double G)
     near(ks_inverse_dt(o, k, fl, inv), speed, 10.0, "speed");
 }
 
+// Reconstruction.hpp:16-37
+double minmod(double l, double r)
+{
+    if (l * r <= 0.0)
+        return 0.0;
+    return l > 0.0 ? std::fmin(l, r) : std::fmax(l, r);
+}
+
+void slopes()
+{
+    const double v[] = {0.0, -0.0, 1.0, -1.0, 1e-12, 1.0 + 1e-15, 2.5, -3e5};
+    auto one = [](double l, double c, double r, double theta) {
+        const double want = minmod(
+            theta * (c - l), minmod(0.5 * (r - l), theta * (r - c)));
+        const double got = limited_slope_f64(l, c, r, theta);
+        check(got == want, "limited slope", got - want);
+    };
+    for (double theta : {0.0, 1.0, 1.3, 2.0})
+    {
+        for (double l : v)
+            for (double c : v)
+                for (double r : v)
+                    one(l, c, r, theta);
+        for (int it = 0; it < 20000; ++it)
+        {
+            const double c = uniform(-1, 1);
+            one(c + uniform(-1, 1) * std::pow(10.0, uniform(-16, 0)), c,
+                c + uniform(-1, 1) * std::pow(10.0, uniform(-16, 0)), theta);
+        }
+    }
+}
+
+// Faces between states that are subsonic, supersonic either way and above
+// the velocity cap, at the floors and far from them.
+void face(double G)
+{
+    const Options o = options(G);
+    Geo g;
+    ks_geo(1.0, uniform(-0.9, 0.9), uniform(2, 20), uniform(-20, 20),
+           uniform(-20, 20), g);
+    Prim side[2];
+    double q[2][5];
+    for (int s = 0; s < 2; ++s)
+    {
+        Prim &p = side[s];
+        p.rho = std::pow(10.0, uniform(-11, 0));
+        p.p = p.rho * std::pow(10.0, uniform(-4, 0));
+        double n[3] = {uniform(-1, 1), uniform(-1, 1), uniform(-1, 1)};
+        const double w = std::sqrt(uniform(0, 0.95) / vsq(n, g.gLL));
+        for (int d = 0; d < 3; ++d)
+            p.v[d] = n[d] * w;
+        q[s][0] = p.rho;
+        q[s][1] = p.p;
+        for (int d = 0; d < 3; ++d)
+            q[s][2 + d] = p.v[d];
+        floors(o, p, g.gLL);
+    }
+    for (int d = 0; d < 3; ++d)
+    {
+        const Cons c[2] = {p2c(side[0], g.gLL), p2c(side[1], g.gLL)};
+        const Cons f[2] = {phys_flux(side[0], c[0], d, g.lapse, g.shift),
+                           phys_flux(side[1], c[1], d, g.lapse, g.shift)};
+        double lo[2], hi[2];
+        for (int s = 0; s < 2; ++s)
+            char_speeds(o, side[s], g, d, lo[s], hi[s]);
+        const double sl = std::fmin(0.0, std::fmin(lo[0], lo[1]));
+        const double su = std::fmax(0.0, std::fmax(hi[0], hi[1]));
+        auto hlle = [&](double fl, double fr, double cl, double cr) {
+            if (sl >= 0.0)
+                return fl;
+            if (su <= 0.0)
+                return fr;
+            return (su * fl - sl * fr + sl * su * (cr - cl)) / (su - sl);
+        };
+        const Cons got =
+            state_flux(make_face_opt<double>(o), q[0], q[1], g, d);
+        // W^2 <= 5 amplifies rounding, at most ten-fold through the speeds
+        const double D = c[0].D + c[1].D;
+        const double E = D + c[0].tau + c[1].tau + side[0].p + side[1].p;
+        near(got.D, hlle(f[0].D, f[1].D, c[0].D, c[1].D), D, "flux D");
+        near(got.tau, hlle(f[0].tau, f[1].tau, c[0].tau, c[1].tau), E,
+             "flux tau");
+        for (int m = 0; m < 3; ++m)
+            near(got.S[m], hlle(f[0].S[m], f[1].S[m], c[0].S[m], c[1].S[m]),
+                 5.0 * E, "flux S");
+    }
+}
+
 // States the recovery meets at its limits.
 void limits(double G)
 {
@@ -161,8 +251,11 @@ int main()
     {
         for (int it = 0; it < 20000; ++it)
             cell(G);
+        for (int it = 0; it < 20000; ++it)
+            face(G);
         limits(G);
     }
+    slopes();
     std::printf("%d failures\n", failures);
     return failures != 0;
 }

@@ -1,5 +1,6 @@
-"""The FP64 Kerr-Schild cell and the recovery's root solve against the general
-functions they replace, on the CPU (tests/ks_cell_check.cu)."""
+"""The FP64 Kerr-Schild cell, the recovery's root solve, the limiter and the
+face flux against the general functions they replace, on the CPU
+(tests/ks_cell_check.cu)."""
 import os
 import subprocess
 
