@@ -637,7 +637,8 @@ def run_widened(hbm_peak):
         "value": cells / (ms / 1e3), "unit": "cell-RHS/s", "ms": ms,
         "fixed_background_rhs_ms": ms_f,
         "hbm_frac": alg / (ms / 1e3) / 1e9 / hbm_peak,
-        "note": "FP64, one thread per cell, each face evaluated by both of its cells (a face-tiled version measured slower)"}
+        "note": "FP64, faces on the shared-memory tiles of the "
+                "fixed-background operator, once each"}
     out["fixed_background_rhs_128"] = {
         "value": cells / (ms_f / 1e3), "unit": "cell-RHS/s", "ms": ms_f,
         "note": "one FP64 compute_rhs of the fixed-background operator "
