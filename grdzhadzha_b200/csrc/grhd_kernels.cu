@@ -44,7 +44,7 @@ __device__ __forceinline__ void record_error(DevStatus *st, int where,
 // Resident blocks per SM the register budget is sized for: the FP32
 // (mixed) kernels fit three 256-thread blocks (80 registers, small
 // spills; measured 13 % faster than two), the FP64 ones two (the FP64 face
-// tile's 108 KB of shared memory allows no more).
+// tile's 111 KB of shared memory allows no more).
 template <typename T> constexpr int kMinBlocks = sizeof(T) == 4 ? 3 : 2;
 
 // The stage kernel's blocks: where its state fits 80 registers with few
