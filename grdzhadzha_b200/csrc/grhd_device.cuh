@@ -1293,21 +1293,23 @@ GRHD_HD __forceinline__ void face_side(const FaceOpt<double> &o,
     s.hi = (base + root) * k - shift;
 }
 
-// The HLLE flux (RiemannSolvers.hpp:69-118) of the two sides, with the
-// weights a = su / (su - sl), b = -sl / (su - sl), ss = sl su / (su - sl):
-// a = 1, b = ss = 0 (up to rounding) where every wave runs right, and the
-// other way round, so the supersonic cases need no branch.
+// The HLLE flux (RiemannSolvers.hpp:69-118) of the two sides.  A comparison
+// with a speed that is not a number keeps the other side's, and where every
+// wave runs one way the flux is the upwind side's alone: frozen primitives of
+// an excised region may be anything, and inside a horizon they must not reach
+// the fluid through a term weighted with zero.
 GRHD_HD __forceinline__ Cons hlle_flux(const FaceSide &l, const FaceSide &r)
 {
-    double sl = l.lo < r.lo ? l.lo : r.lo;
-    double su = l.hi > r.hi ? l.hi : r.hi;
-    sl = sl < 0.0 ? sl : 0.0;
-    su = su > 0.0 ? su : 0.0;
-    const double w = su - sl;
-    const double inv = w > 0.0 ? rcp_ulp(w) : 0.0;
-    // both speeds zero: the left flux, as the reference's first branch
-    const double a = w > 0.0 ? su * inv : 1.0;
-    const double b = -sl * inv, ss = sl * a;
+    double sl = l.lo < 0.0 ? l.lo : 0.0;
+    double su = l.hi > 0.0 ? l.hi : 0.0;
+    sl = r.lo < sl ? r.lo : sl;
+    su = r.hi > su ? r.hi : su;
+    if (!(sl < 0.0))
+        return l.f;
+    if (!(su > 0.0))
+        return r.f;
+    const double inv = rcp_ulp(su - sl);
+    const double a = su * inv, b = -sl * inv, ss = sl * a;
     Cons f;
     f.D = a * l.f.D + b * r.f.D + ss * (r.c.D - l.c.D);
     f.tau = a * l.f.tau + b * r.f.tau + ss * (r.c.tau - l.c.tau);

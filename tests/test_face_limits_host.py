@@ -1,0 +1,17 @@
+"""The FP64 face flux next to states that are not numbers or not finite, on
+the CPU (tests/face_limits_check.cu)."""
+import os
+import subprocess
+
+from grdzhadzha_b200 import build as B
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+def test_face_flux_beside_frozen_states(tmp_path):
+    exe = str(tmp_path / "face_limits_check")
+    subprocess.run([B.nvcc(), "-std=c++17", "-O2", "-I", B.CSRC, "-Xcompiler",
+                    "-ffp-contract=off", "-o", exe,
+                    os.path.join(HERE, "face_limits_check.cu")], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout
