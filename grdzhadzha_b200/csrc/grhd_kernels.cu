@@ -821,6 +821,7 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
     const bool col_ok = ci <= b.hi[0] && cj <= b.hi[1];
     const int64_t plane = (int64_t)b.gn[0] * b.gn[1];
     const int own_p = (bb + 2) * kPW + a + 2, own_g = (bb + 1) * kGW + a + 1;
+    const int reach = fo.reach;
     // primitive tiles of planes k0-1, k0 and k0+1; P0, P1, P2 hold the planes
     // k, k+1, k+2 of the march
     T *P0 = P, *P1 = P + 5 * nP, *P2 = P + 2 * 5 * nP;
@@ -835,7 +836,8 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
         T unused[5];
         cell_states(fo, load_pv_global<T, CG>(pcol, b.pcs, 0),
                     load_pv_global<T, CG>(pcol, b.pcs, plane),
-                    load_pv_global<T, CG>(pcol, b.pcs, 2 * plane), unused, up);
+                    load_pv_global<T, CG>(pcol, b.pcs, (1 + reach) * plane),
+                    unused, up);
     }
 
     ConsT<T> Flo = zero_cons<T>();
@@ -862,9 +864,9 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
                 geo_sum(G, nG, (fb + 1) * kGW + fa, (fb + 1) * kGW + fa + 1, 0,
                         gf);
                 const ConsT<T> f = face_flux(
-                    fo, load_pv_smem(P0, row), load_pv_smem(P0, row + 1),
-                    load_pv_smem(P0, row + 2), load_pv_smem(P0, row + 3), gf,
-                    0);
+                    fo, load_pv_smem(P0, row + 1 - reach),
+                    load_pv_smem(P0, row + 1), load_pv_smem(P0, row + 2),
+                    load_pv_smem(P0, row + 2 + reach), gf, 0);
                 const int fi = fb * wX + fa;
                 if (MDOT && fa < kTC && i0 + fa <= b.hi[0])
                     macc +=
@@ -889,9 +891,10 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
                 geo_sum(G, nG, fb * kGW + fa + 1, (fb + 1) * kGW + fa + 1, 1,
                         gf);
                 const ConsT<T> f = face_flux(
-                    fo, load_pv_smem(P0, col), load_pv_smem(P0, col + kPW),
+                    fo, load_pv_smem(P0, col + (1 - reach) * kPW),
+                    load_pv_smem(P0, col + kPW),
                     load_pv_smem(P0, col + 2 * kPW),
-                    load_pv_smem(P0, col + 3 * kPW), gf, 1);
+                    load_pv_smem(P0, col + (2 + reach) * kPW), gf, 1);
                 const int fi = fb * kTC + fa;
                 if (MDOT && fb < kTC && j0 + fb <= b.hi[1])
                     macc +=
@@ -952,7 +955,7 @@ faces_tile(const T *__restrict__ prim, const T *__restrict__ src,
             geo_sum_z(G, nG, own_g, gn, gf);
             T low[5], next[5];
             cell_states(fo, w1, load_pv_smem(P1, own_p),
-                        load_pv_smem(P2, own_p), low, next);
+                        load_pv_smem(reach ? P2 : P1, own_p), low, next);
             Fhi = state_flux(fo, up, low, gf, 2);
 #pragma unroll
             for (int c = 0; c < 5; ++c)
