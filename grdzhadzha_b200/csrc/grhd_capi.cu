@@ -41,6 +41,7 @@ struct grhd_ctx
     size_t ccz4_geo_cap = 0;
     double *ccz4_stage = nullptr; // CCZ4 operator: SSPRK2 stage (GRHD)
     size_t ccz4_stage_cap = 0;
+    int max_pitch = 0;            // of a pitched copy, bytes
     double *host_state = nullptr; // device copy of a host-held state
     size_t host_state_cap = 0;
     double *prim2 = nullptr; // host-buffer step: second primitive cache
@@ -556,6 +557,8 @@ int grhd_create(const grhd_params *params, grhd_ctx **out)
     ctx->opt = make_options(*params);
     std::memset(&ctx->last_error, 0, sizeof(ctx->last_error));
     if (cudaGetDevice(&ctx->device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&ctx->max_pitch, cudaDevAttrMaxPitch,
+                               ctx->device) != cudaSuccess ||
         configure_kernels() != cudaSuccess ||
         cudaMalloc((void **)&ctx->status, sizeof(DevStatus)) != cudaSuccess ||
         cudaMallocHost((void **)&ctx->status_h, sizeof(DevStatus)) !=
@@ -1061,14 +1064,16 @@ int pipe_setup(grhd_ctx *ctx, int nchunks)
 // `bytes` of each of `rows` components (stride cs on both sides).  A pitched
 // copy of long rows saves the gaps between as many copies (a host step of
 // 161 x 143 x 127, rows of 1.5 MB: 8.0 -> 7.5 ms); with short rows (96^3, 0.6
-// MB: 2.91 against 2.98) separate copies are the faster.
-cudaError_t copy_components(double *dst, const double *src, size_t cs,
-                            size_t bytes, int rows, cudaMemcpyKind kind,
-                            cudaStream_t s)
+// MB: 2.91 against 2.98) separate copies are the faster.  So goes a stride
+// above the largest pitch that is documented for the device (2^31 - 1 bytes,
+// a box of 646^3 cells), which drivers may refuse.
+cudaError_t copy_components(const grhd_ctx *ctx, double *dst,
+                            const double *src, size_t cs, size_t bytes,
+                            int rows, cudaMemcpyKind kind, cudaStream_t s)
 {
-    if (bytes >= (size_t)1 << 20)
-        return cudaMemcpy2DAsync(dst, cs * sizeof(double), src,
-                                 cs * sizeof(double), bytes, rows, kind, s);
+    const size_t pitch = cs * sizeof(double);
+    if (bytes >= (size_t)1 << 20 && pitch <= (size_t)ctx->max_pitch)
+        return cudaMemcpy2DAsync(dst, pitch, src, pitch, bytes, rows, kind, s);
     cudaError_t e = cudaSuccess;
     for (int q = 0; q < rows && e == cudaSuccess; ++q)
         e = cudaMemcpyAsync(dst + q * cs, src + q * cs, bytes, kind, s);
@@ -1119,7 +1124,7 @@ int enqueue_rk4_host_pipelined(grhd_ctx *ctx, double *host, double *dev,
             const size_t bytes =
                 (size_t)(q1 - q0 + 1) * plane * sizeof(double);
             in += (long long)(bytes * (last - first));
-            return copy_components(dev + at, host + at, cs, bytes,
+            return copy_components(ctx, dev + at, host + at, cs, bytes,
                                    last - first, cudaMemcpyHostToDevice,
                                    ctx->h2d);
         };
@@ -1196,7 +1201,7 @@ int enqueue_rk4_host_pipelined(grhd_ctx *ctx, double *host, double *dev,
                 const size_t off = (size_t)(z.plo(j) - b.glo[2]) * plane;
                 const size_t n = (size_t)(z.phi(j) - z.plo(j) + 1) * plane;
                 GRHD_CUDA(ctx, copy_components(
-                                   host + off, dev + off, cs,
+                                   ctx, host + off, dev + off, cs,
                                    n * sizeof(double), kStateComps,
                                    cudaMemcpyDeviceToHost, ctx->d2h));
                 out += (long long)(n * sizeof(double) * kStateComps);
