@@ -113,15 +113,18 @@ void member_tiles(const BoxDev &b, int zchunk, int t[3])
 // The launch shape until the autotuner or the caller sets another: every
 // block that fits, since the phases wait on latency (24 mixed members of
 // 32..96 cells a side, two steps: 50.4 ms with one block per SM, 23.8 with
-// three), and of 32, 16, 8 and 4 planes a face tile the count whose tiles
-// fill the fewest waves of blocks (a tile costs its planes and 0.7 of one;
-// five members of 32..48: 4.9 ms with 32 planes, 1.5 with 4).
+// three), and of 32, 16 and 8 planes a face tile the count whose tiles fill
+// the fewest waves of blocks (a tile costs its planes and 0.7 of one; a step
+// of five FP64 members of at most 56 x 56 x 9 cells: 1.46 ms with 32 planes,
+// 0.54 with 8).  The shape is one that the autotuner tries, which therefore never
+// leaves a slower one; 4 planes (0.37 ms there) are not, and remain the
+// caller's to set.
 grhd_ensemble_tuning default_tuning(const grhd_ensemble *e)
 {
     grhd_ensemble_tuning best = {32, e->max_bps, 0.0};
     const int64_t slots = (int64_t)e->max_bps * e->num_sms;
     double best_cost = 0.0;
-    for (int z : {32, 16, 8, 4})
+    for (int z : {32, 16, 8})
     {
         int64_t tiles = 0;
         for (const EnsMember &d : e->desc)

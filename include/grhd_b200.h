@@ -702,9 +702,9 @@ int grhd_ensemble_get_tuning(const grhd_ensemble *ens,
 int grhd_ensemble_set_tuning(grhd_ensemble *ens,
                              const grhd_ensemble_tuning *tuning);
 /* Times `trial_steps` steps of every candidate launch shape (z chunks 8,
- * 16, 32, 64 x 1..max blocks per SM) on the real members, keeps the
- * fastest and restores the states, times, accretion integrals and
- * counters as they were. */
+ * 16, 32, 64 x 1..max blocks per SM; a new ensemble's shape is one of
+ * them) on the real members, keeps the fastest and restores the states,
+ * times, accretion integrals and counters as they were. */
 int grhd_ensemble_autotune(grhd_ensemble *ens, int trial_steps,
                            grhd_ensemble_tuning *best, void *stream);
 /* `steps` RK4 steps of every member in one launch; use_graph = 1 replays a
