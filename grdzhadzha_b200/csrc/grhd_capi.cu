@@ -1763,6 +1763,14 @@ int grhd_face_zchunk(int nx, int ny, int nz, int resident_blocks,
     return GRHD_OK;
 }
 
+int grhd_face_march(int nx, int ny, int nz, int resident_blocks, int *planes)
+{
+    if (nx < 1 || ny < 1 || nz < 1 || resident_blocks < 1 || !planes)
+        return GRHD_ERR_INVALID_ARG;
+    *planes = face_march(nx, ny, nz, resident_blocks);
+    return GRHD_OK;
+}
+
 int grhd_eval_arith(grhd_ctx *ctx, int64_t n, const double *a,
                     const double *b, double *out, void *stream)
 {

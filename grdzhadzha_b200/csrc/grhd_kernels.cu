@@ -2795,23 +2795,19 @@ int64_t face_makespan(int64_t nf, int64_t df, int64_t np, int64_t dp,
 // Marches down to one plane spread a small box over the idle SMs: a plane
 // takes one block about 9 us, whatever the box (a 16^3 right-hand side:
 // 102 us with at least four planes a block, 58 with one; 45x38x31: 84, 70).
-int face_zchunk(const BoxDev &b, int zchunk, bool fp32)
+int face_march(int nx, int ny, int nz, int64_t slots)
 {
-    if (zchunk > 0)
-        return zchunk;
-    const int64_t slots = face_slots(fp32);
-    const int64_t tiles = (int64_t)((b.in[0] + kTC - 1) / kTC) *
-                          ((b.in[1] + kTC - 1) / kTC);
+    const int64_t tiles =
+        (int64_t)((nx + kTC - 1) / kTC) * ((ny + kTC - 1) / kTC);
     const int cand[] = {48, 40, 32, 24, 20, 16, 13, 12, 11, 10,
                         9,  8,  7,  6,  5,  4,  3,  2,  1};
     int best = 1;
     int64_t best_cost = -1;
     for (int z : cand)
     {
-        const int r = b.in[2] % z;
-        const int64_t cost =
-            face_makespan(tiles * (b.in[2] / z), 10 * z + 7, r ? tiles : 0,
-                          10 * r + 7, slots);
+        const int r = nz % z;
+        const int64_t cost = face_makespan(tiles * (nz / z), 10 * z + 7,
+                                           r ? tiles : 0, 10 * r + 7, slots);
         if (best_cost < 0 || cost < best_cost)
         {
             best = z;
@@ -2819,6 +2815,13 @@ int face_zchunk(const BoxDev &b, int zchunk, bool fp32)
         }
     }
     return best;
+}
+
+int face_zchunk(const BoxDev &b, int zchunk, bool fp32)
+{
+    return zchunk > 0 ? zchunk
+                      : face_march(b.in[0], b.in[1], b.in[2],
+                                   face_slots(fp32));
 }
 
 int face_zchunk_model(int nx, int ny, int nz, int64_t slots)

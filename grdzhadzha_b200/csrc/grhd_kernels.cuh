@@ -138,9 +138,12 @@ constexpr int kGeoFields = 13; // gamma_ij, diag gamma^ij, lapse, shift
 // Per-device kernel attributes (dynamic shared memory of the face kernels).
 cudaError_t configure_kernels();
 // z-march length (planes per block) of the face kernel for box b: zchunk
-// when positive, else the length whose launch finishes first (the RHS does
-// not depend on it).
+// when positive, else face_march on the device's resident face blocks (the
+// RHS does not depend on it).
 int face_zchunk(const BoxDev &b, int zchunk, bool fp32);
+// The length whose launch finishes first on `slots` resident blocks.  Host
+// only.
+int face_march(int nx, int ny, int nz, int64_t slots);
 // The C entry point's schedule estimate, for tiles of 15 cells and of 32,
 // 16, 8, 6 and 4 planes: the length with the shortest makespan when the
 // launch's blocks -- every full z block of every (x,y) tile, then the short

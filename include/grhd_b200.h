@@ -334,12 +334,21 @@ int grhd_eval_con2prim(grhd_ctx *ctx, int64_t n, const double *cons,
  * interior cut into 15 x 15-cell columns on a device with `resident_blocks`
  * blocks resident at once (SMs x blocks per SM): of 32, 16, 8, 6 and 4
  * planes, the one whose blocks list-scheduled in launch order finish first,
- * a block costing its planes plus two lead-in planes.  The face kernel's own
- * launches schedule its 16 x 16-cell tiles the same way with finer costs and
- * lengths; the RHS does not depend on the length.  Host only (no device
- * call).  New (the reference has no face kernel). */
+ * a block costing its planes plus two lead-in planes.  No kernel has that
+ * tiling: it is kept for its callers; what the launches take is
+ * grhd_face_march.  Host only (no device call).  New (the reference has no
+ * face kernel). */
 int grhd_face_zchunk(int nx, int ny, int nz, int resident_blocks,
                      int *zchunk);
+
+/* The face pass's z-march length (planes per block) for an nx x ny x nz
+ * interior on a device with `resident_blocks` face blocks resident at once
+ * (SMs x blocks per SM): of 19 lengths from 48 planes to one, the one whose
+ * blocks -- 16 x 16-cell columns, list-scheduled in launch order -- finish
+ * first, a block costing its planes plus 0.7 of one.  The kernels choose it
+ * this way whenever their caller gives no z-march length; the RHS does not
+ * depend on it.  Host only (no device call).  New. */
+int grhd_face_march(int nx, int ny, int nz, int resident_blocks, int *planes);
 
 /* The FP64 division, reciprocal, square root and reciprocal square root
  * the kernels compute with, at n points: out[4n] = (a/b, 1/b, sqrt(a),
