@@ -143,9 +143,10 @@ GRHD_HD __forceinline__ void p2c_rev(const Prim &pr, const double G[6],
 // enforce_primitive_floors, Atmosphere.hpp:24-46.  `in` is the input of
 // the floors (eps unused: the floors recompute it); `ob` the adjoint of
 // their output (eps included); adds the adjoint of rho, p, v of the input.
+// v2 is the squared velocity that the forward compared with the cap.
 GRHD_HD __forceinline__ void floors_rev(const Options &o, const Prim &in,
-                               const double G[6], const PrimBar &ob,
-                               PrimBar &ib, double Gbar[6])
+                               const double G[6], double v2,
+                               const PrimBar &ob, PrimBar &ib, double Gbar[6])
 {
     const double rho1 = fmax(in.rho, o.rho_floor);
     const double p1 = fmax(in.p, o.p_floor);
@@ -158,7 +159,6 @@ GRHD_HD __forceinline__ void floors_rev(const Options &o, const Prim &in,
         ib.rho += rho1bar;
     if (in.p > o.p_floor)
         ib.p += p1bar;
-    const double v2 = vsq(in.v, G);
     if (v2 >= o.atmo_vmax2)
     {
         const double s = sqrt_(div_(o.atmo_vmax2, v2));
@@ -173,6 +173,13 @@ GRHD_HD __forceinline__ void floors_rev(const Options &o, const Prim &in,
         for (int k = 0; k < 3; ++k)
             ib.v[k] += ob.v[k];
     }
+}
+
+GRHD_HD __forceinline__ void floors_rev(const Options &o, const Prim &in,
+                               const double G[6], const PrimBar &ob,
+                               PrimBar &ib, double Gbar[6])
+{
+    floors_rev(o, in, G, vsq(in.v, G), ob, ib, Gbar);
 }
 
 // compute_flux, Valencia.hpp:230-259
@@ -562,7 +569,7 @@ GRHD_HD inline void con2prim_rev(const Options &o, const Cons &c,
 }
 
 // The primitives of recover_primitive at a known converged pressure p
-// (c2p_finish without the velocity check).
+// (c2p_finish_gUU without the velocity check).
 GRHD_HD inline Prim c2p_at(const Options &o, const Cons &c,
                            const double gUU[6], double p)
 {
@@ -578,6 +585,18 @@ GRHD_HD inline Prim c2p_at(const Options &o, const Cons &c,
     out.v[0] = (gUU[0] * c.S[0] + gUU[1] * c.S[1] + gUU[2] * c.S[2]) * ie;
     out.v[1] = (gUU[1] * c.S[0] + gUU[3] * c.S[1] + gUU[4] * c.S[2]) * ie;
     out.v[2] = (gUU[2] * c.S[0] + gUU[4] * c.S[1] + gUU[5] * c.S[2]) * ie;
+    return out;
+}
+
+// The primitives that ks_con2prim found at its converged pressure p, bit for
+// bit: the same operations, every one of them rounded by itself.
+GRHD_HD inline Prim ks_c2p_at(const Options &o, const KsCell &k, const Cons &c,
+                              double p)
+{
+    double mU[3];
+    Prim out;
+    ks_raise(k, c.S, mU);
+    c2p_finish(o, c, mU, dot3(c.S, mU), p, out);
     return out;
 }
 
@@ -789,22 +808,30 @@ GRHD_HD inline bool differs(const Prim &a, const Prim &b)
 // (recover_primitives_and_apply_atmosphere_from_fixed_background,
 // FixedBGFArrayBoxFiniteVolume.hpp:60-110) as recorded by the forward
 // sweep: branch 0 kept the updated state Y, 1 replaced it by p2c of the
-// floored con2prim result (converged pressure pY), 2 by the atmosphere.
+// floored con2prim result (converged pressure pY), 2 by the atmosphere.  With
+// the Kerr-Schild cell k, which the forward recovers on, the primitives and
+// the squared velocity are its own bit for bit, so that every floor decides
+// as it did (a reset cell's density sits on the floor to within an ulp).
 GRHD_HD inline ConsBar recovery_rev(const Options &o, const Cons &Y, int br,
                                     double pY, const Geo &g,
-                                    const ConsBar &Ub, GeoBar &gb)
+                                    const ConsBar &Ub, GeoBar &gb,
+                                    const KsCell *k = nullptr)
 {
     if (br == 0)
         return Ub;
     ConsBar Yb = zero_cons_bar();
     if (br != 1)
         return Yb;
-    const Prim pr = c2p_at(o, Y, g.gUU, pY);
+    const Prim pr = k ? ks_c2p_at(o, *k, Y, pY) : c2p_at(o, Y, g.gUU, pY);
     Prim fl = pr;
-    floors(o, fl, g.gLL);
+    if (k)
+        ks_floors(o, *k, fl);
+    else
+        floors(o, fl, g.gLL);
     PrimBar flb = zero_prim_bar(), prb = zero_prim_bar();
     p2c_rev(fl, g.gLL, Ub, flb, gb.gLL);
-    floors_rev(o, pr, g.gLL, flb, prb, gb.gLL);
+    floors_rev(o, pr, g.gLL, k ? ks_vsq(*k, pr.v) : vsq(pr.v, g.gLL), flb,
+               prb, gb.gLL);
     con2prim_rev(o, Y, g.gUU, pY, prb, Yb, gb.gUU);
     return Yb;
 }

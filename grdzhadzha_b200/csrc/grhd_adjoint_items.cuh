@@ -556,7 +556,10 @@ __host__ __device__ inline double cell_rev_item(const AdjRhs &A,
             Y.S[1] = S.Y[2 * rcs + t];
             Y.S[2] = S.Y[3 * rcs + t];
             Y.tau = S.Y[4 * rcs + t];
-            B = recovery_rev(o, Y, S.br[t], S.pY[t], ge, Ub, gb);
+            KsCell kc;
+            if (S.br[t] == 1)
+                ks_cell(A.M, A.a, x, y, z, kc);
+            B = recovery_rev(o, Y, S.br[t], S.pY[t], ge, Ub, gb, &kc);
         }
         const double Bv[5] = {B.D, B.S[0], B.S[1], B.S[2], B.tau};
         // lambda_k of the previous stage: cA A + cB B
@@ -627,7 +630,10 @@ __host__ __device__ inline double proj_rev_item(
     values_of(gd, g);
     GeoBar gb;
     zero(gb);
-    const ConsBar B = recovery_rev(o, Yc, br[t], pY[t], g, Ub, gb);
+    KsCell kc;
+    if (br[t] == 1)
+        ks_cell(M, a, x, y, z, kc);
+    const ConsBar B = recovery_rev(o, Yc, br[t], pY[t], g, Ub, gb, &kc);
     const double Bv[5] = {B.D, B.S[0], B.S[1], B.S[2], B.tau};
     for (int q = 0; q < 5; ++q)
     {

@@ -113,18 +113,15 @@ GRHD_HD inline PrimT<Dual> con2prim_tan(const Options &o, const ConsT<Dual> &c,
 }
 
 // enforce_primitive_floors (Atmosphere.hpp:24-46) in tangent form; `in`
-// holds the double input on which floors_rev decides (eps unused).
+// holds the double input and v2 its squared velocity, on which floors_rev
+// decides (eps unused).
 GRHD_HD inline PrimT<Dual> floors_tan(const Options &o, const Prim &in,
-                                      const PrimT<Dual> &ind,
+                                      double v2, const PrimT<Dual> &ind,
                                       const Dual G[6])
 {
     PrimT<Dual> out;
     out.rho = in.rho > o.rho_floor ? ind.rho : Dual(fmax(in.rho, o.rho_floor));
     out.p = in.p > o.p_floor ? ind.p : Dual(fmax(in.p, o.p_floor));
-    double Gv[6];
-    for (int q = 0; q < 6; ++q)
-        Gv[q] = G[q].v;
-    const double v2 = vsq(in.v, Gv);
     if (v2 >= o.atmo_vmax2)
     {
         const Dual v2d = vsq(ind.v, G);
@@ -137,6 +134,16 @@ GRHD_HD inline PrimT<Dual> floors_tan(const Options &o, const Prim &in,
             out.v[k] = ind.v[k];
     out.eps = out.p / ((o.G - 1.0) * out.rho);
     return out;
+}
+
+GRHD_HD inline PrimT<Dual> floors_tan(const Options &o, const Prim &in,
+                                      const PrimT<Dual> &ind,
+                                      const Dual G[6])
+{
+    double Gv[6];
+    for (int q = 0; q < 6; ++q)
+        Gv[q] = G[q].v;
+    return floors_tan(o, in, vsq(in.v, Gv), ind, G);
 }
 
 // rad of compute_characteristic_speeds in double, computed as
@@ -271,12 +278,13 @@ GRHD_HD inline ConsT<Dual> face_flux_tan(
 }
 
 // The post-update recovery of one cell in tangent form, with the branch
-// the forward sweep recorded (recovery_rev transposed): 0 kept Y, 1
-// replaced it by p2c of the floored con2prim result at pressure pY, 2 by
-// the atmosphere (v = 0: p2c of it does not depend on the metric).
+// the forward sweep recorded (recovery_rev transposed, deciding on the
+// Kerr-Schild cell k as it does): 0 kept Y, 1 replaced it by p2c of the
+// floored con2prim result at pressure pY, 2 by the atmosphere (v = 0: p2c of
+// it does not depend on the metric).
 GRHD_HD inline ConsT<Dual> recovery_tan(const Options &o, const ConsT<Dual> &Y,
                                         int br, double pY,
-                                        const GeoT<Dual> &g)
+                                        const GeoT<Dual> &g, const KsCell &k)
 {
     if (br == 0)
         return Y;
@@ -293,8 +301,8 @@ GRHD_HD inline ConsT<Dual> recovery_tan(const Options &o, const ConsT<Dual> &Y,
         return z;
     }
     const PrimT<Dual> pr = con2prim_tan(o, Y, g.gUU, pY);
-    const Prim prv = c2p_at(o, values_of(Y), gv.gUU, pY);
-    const PrimT<Dual> fl = floors_tan(o, prv, pr, g.gLL);
+    const Prim prv = ks_c2p_at(o, k, values_of(Y), pY);
+    const PrimT<Dual> fl = floors_tan(o, prv, ks_vsq(k, prv.v), pr, g.gLL);
     return p2c(fl, g.gLL);
 }
 
@@ -578,7 +586,9 @@ __host__ __device__ inline void tan_stage_item(
     GeoT<Dual> gd;
     ks_metric_spin<false>(M, a, x, y, z, gd, nullptr);
     scale_tangent(gd, da);
-    const ConsT<Dual> U = recovery_tan(o, Yd, br[t], pY[t], gd);
+    KsCell kc;
+    ks_cell(M, a, x, y, z, kc);
+    const ConsT<Dual> U = recovery_tan(o, Yd, br[t], pY[t], gd, kc);
     out[0 * b.rcs + t] = U.D.d;
     for (int m = 0; m < 3; ++m)
         out[(1 + m) * b.rcs + t] = U.S[m].d;
