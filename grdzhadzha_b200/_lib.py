@@ -206,6 +206,7 @@ SIGNATURES = {
     "grhd_eval_con2prim": (C.c_int, [_vp, C.c_int64, _vp, _vp, _vp, _vp, _vp,
                                      _vp, _vp]),
     "grhd_eval_arith": (C.c_int, [_vp, C.c_int64, _vp, _vp, _vp, _vp]),
+    "grhd_eval_arith_ulp": (C.c_int, [_vp, C.c_int64, _vp, _vp, _vp]),
     "grhd_face_zchunk": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int,
                                    C.POINTER(C.c_int)]),
     "grhd_face_march": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int,

@@ -38,8 +38,7 @@ __host__ __device__ constexpr int sym(int i, int j)
 // normal numbers up to 2^1021, and 0 for the square root; a zero divisor
 // or a quotient that overflows gives NaN (not +-inf), and a subnormal
 // operand is flushed to zero.  The oracle and the host keep IEEE
-// division, as does the binary's volume-time source (pn_scalar), whose
-// time difference is rounded as the reference's.  FP32: the SFU
+// division.  FP32: the SFU
 // reciprocal / reciprocal square root (a few ulp), which is what makes the
 // FP32 path cheap.
 
@@ -136,7 +135,8 @@ GRHD_HD __forceinline__ double mul_(double a, double b)
     return a * b;
 #endif
 }
-// 1/a and 1/sqrt(a) within about one ulp: one step of
+// 1/a within 0.51 ulp and 1/sqrt(a) within 1.02 (grhd_eval_arith_ulp's test):
+// one step of
 // the third-order iteration (Householder's) from the approximate value y0 of
 // relative error d <= 2^-20: with e = 1 - a y0, 1/a = y0 (1 + e + e^2) up to
 // d^3; with e = 1 - a y0^2, a^-1/2 = y0 (1 + e/2 + 3 e^2/8) up to d^3.  Three

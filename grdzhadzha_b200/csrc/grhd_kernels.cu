@@ -1844,6 +1844,16 @@ __global__ void k_eval_arith(int64_t n, const double *__restrict__ a,
     out[4 * t + 3] = rsqrt_(a[t]);
 }
 
+__global__ void k_eval_arith_ulp(int64_t n, const double *__restrict__ a,
+                                 double *__restrict__ out)
+{
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t >= n)
+        return;
+    out[2 * t] = rcp_ulp(a[t]);
+    out[2 * t + 1] = rsqrt_ulp(a[t]);
+}
+
 // ------------------------------------------------------------- ensemble
 
 __device__ __forceinline__ unsigned long long global_ns()
@@ -3064,6 +3074,13 @@ void launch_eval_arith(int64_t n, const double *a, const double *b,
     if (n <= 0)
         return;
     k_eval_arith<<<(int)((n + 255) / 256), 256, 0, s>>>(n, a, b, out);
+}
+
+void launch_eval_arith_ulp(int64_t n, const double *a, double *out,
+                           cudaStream_t s)
+{
+    if (n > 0)
+        k_eval_arith_ulp<<<(int)((n + 255) / 256), 256, 0, s>>>(n, a, out);
 }
 
 void launch_ccz4_fill(double *m, int64_t mcs, double *q, int64_t qcs,

@@ -228,6 +228,8 @@ void launch_eval_con2prim(int64_t n, const double *cons, const double *gUU,
                           double *resid, cudaStream_t s);
 void launch_eval_arith(int64_t n, const double *a, const double *b,
                        double *out, cudaStream_t s);
+void launch_eval_arith_ulp(int64_t n, const double *a, double *out,
+                           cudaStream_t s);
 
 // ------------------------------------------------------------ ensemble
 // Many independent boxes (members) advanced by one persistent launch: each

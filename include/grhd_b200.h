@@ -358,6 +358,13 @@ int grhd_face_march(int nx, int ny, int nz, int resident_blocks, int *planes);
  * uses IEEE operations).  Device pointers. */
 int grhd_eval_arith(grhd_ctx *ctx, int64_t n, const double *a,
                     const double *b, double *out, void *stream);
+/* The FP64 reciprocal and reciprocal square root of the face fluxes, the
+ * root solve and the Kerr-Schild cell, at n points: out[2n] = (1/a,
+ * 1/sqrt(a)) per point, the first within 0.51 and the second within 1.02
+ * units in the last place of the exact value for normal operands and
+ * results.  New.  Device pointers. */
+int grhd_eval_arith_ulp(grhd_ctx *ctx, int64_t n, const double *a,
+                        double *out, void *stream);
 
 /* ---- initial data (setup, not part of a step) ---- */
 
