@@ -1358,25 +1358,24 @@ template <typename T> struct StageIn
 static_assert(kD == 0 && kS1 == 1 && kTau == 4,
               "the conserved components come first, in the RHS's order");
 
-template <int MODE, typename T, bool CG>
+// The ensemble's loads of an RK4 stage.
+template <typename T>
 __device__ __forceinline__ void
-stage_load(StageIn<T> &in, const double *un, int64_t ucs, const double *us,
-           int64_t tcs, const T *__restrict__ kv,
-           const double *__restrict__ acc, const T *__restrict__ prim_in,
-           const BoxDev &b, int stage, int64_t g, int64_t t)
+stage_load(StageIn<T> &in, const double *un, int64_t ucs,
+           const T *__restrict__ kv, const double *__restrict__ acc,
+           const T *__restrict__ prim_in, const BoxDev &b, int stage,
+           int64_t g, int64_t t)
 {
 #pragma unroll
     for (int c = 0; c < 5; ++c)
     {
-        in.u[c] = rd<CG>(&un[c * ucs + g]);
-        in.k[c] = rd<CG>(&kv[c * b.rcs + t]);
-        if (MODE == 0 && stage > 0)
-            in.v[c] = rd<CG>(&acc[c * b.rcs + t]);
-        if (MODE == 2)
-            in.v[c] = rd<CG>(&us[c * tcs + g]);
+        in.u[c] = rd<true>(&un[c * ucs + g]);
+        in.k[c] = rd<true>(&kv[c * b.rcs + t]);
+        if (stage > 0)
+            in.v[c] = rd<true>(&acc[c * b.rcs + t]);
     }
     if (sizeof(T) != sizeof(double))
-        in.p = prim_in ? rd<CG>(&prim_in[1 * b.pcs + g]) : T(0);
+        in.p = prim_in ? rd<true>(&prim_in[1 * b.pcs + g]) : T(0);
 }
 
 template <int MODE, typename T, bool CG = false, int BGK = -1>
@@ -2145,10 +2144,10 @@ __global__ void __launch_bounds__(kEnsItemCells, kMinBlocks<T>)
                         interior_cell(ms.b, t, ic, jc, kc);
                         const int64_t g = ms.b.gidx(ic, jc, kc);
                         StageIn<T> in;
-                        stage_load<0, T, true>(
-                            in, ms.state, ms.b.cs, nullptr, 0,
-                            static_cast<const T *>(ms.k), ms.acc,
-                            static_cast<const T *>(ms.prim), ms.b, s, g, t);
+                        stage_load(in, ms.state, ms.b.cs,
+                                   static_cast<const T *>(ms.k), ms.acc,
+                                   static_cast<const T *>(ms.prim), ms.b, s,
+                                   g, t);
                         stage_item<0, T, true, kEnsBgk>(
                             in, ms.state, ms.b.cs, s < 3 ? ms.stage : ms.state,
                             s < 3 ? ms.sb.cs : ms.b.cs, ms.acc,
