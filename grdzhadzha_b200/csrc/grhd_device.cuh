@@ -883,8 +883,13 @@ GRHD_HD __forceinline__ bool c2p_solve(const Options &o, const Cons &c,
     const bool at_floor = fabs(f_lower) <= tol;
     if (!(f_lower < 0.0) && !at_floor)
     {
-        // no root above the floor (or not a number)
-        resid = f_lower >= 0.0 ? 0.0 : f_lower;
+        // no root above the floor, or not a number: every iteration of the
+        // reference's loop stays at the floor
+        if (!(f_lower >= 0.0))
+        {
+            iters = o.rec_maxit;
+            resid = f_lower;
+        }
         return false;
     }
     const bool bracketed = f_lower < 0.0;
