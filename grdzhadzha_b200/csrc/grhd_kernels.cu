@@ -2736,6 +2736,26 @@ template cudaError_t launch_ensemble<float>(const EnsLaunch &, int,
 
 namespace
 {
+// SMs of the current device (a B200's 148 where it cannot be asked)
+int num_sms()
+{
+    static std::atomic<int> cache[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64)
+        return 148;
+    int have = cache[dev].load(std::memory_order_relaxed);
+    if (have > 0)
+        return have;
+    if (cudaDeviceGetAttribute(&have, cudaDevAttrMultiProcessorCount, dev) !=
+        cudaSuccess)
+    {
+        (void)cudaGetLastError();
+        return 148;
+    }
+    cache[dev].store(have, std::memory_order_relaxed);
+    return have;
+}
+
 // resident face-kernel blocks of the current device (SMs x blocks per SM
 // at the kernel's registers and shared memory), per precision
 int face_slots(bool fp32)
@@ -2743,13 +2763,13 @@ int face_slots(bool fp32)
     static std::atomic<int> cache[64][2];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64)
-        return fp32 ? 3 * 148 : 2 * 148;
+        return (fp32 ? 3 : 2) * num_sms();
     std::atomic<int> &c = cache[dev][fp32 ? 1 : 0];
     const int have = c.load(std::memory_order_relaxed);
     if (have > 0)
         return have;
-    int sms = 148, per = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = num_sms();
+    int per = 0;
     const cudaError_t e =
         fp32 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                    &per, k_faces<float, false, 0>, kTB * kTB,
@@ -2910,7 +2930,7 @@ bool launch_prepare(double *state, double *prim, double *src, const BoxDev &b,
     const int64_t nshell = b.gvol() - b.ivol();
     // a box with more cells than the SMs hold at once fills them with either
     // pass alone, and the separate ones keep three blocks per SM
-    if (b.ivol() + nshell > 148 * 2 * 256 * 4)
+    if (b.ivol() + nshell > (int64_t)num_sms() * 2 * 256 * 4)
         return false;
     const int ghosts = (int)((nshell + 255) / 256);
     const int grid = ghosts + (int)((b.ivol() + 255) / 256);
@@ -2976,7 +2996,7 @@ template <typename T> int stage_grid(int64_t n, int kind)
 {
     const int64_t blocks = (n + kStageThreads - 1) / kStageThreads;
     const int per = kind == 1 ? kStageBlocks<T, 1> : kStageBlocks<T, 0>;
-    return (int)(blocks >= 8 * 148 * per ? (blocks + 1) / 2 : blocks);
+    return (int)(blocks >= 8 * num_sms() * per ? (blocks + 1) / 2 : blocks);
 }
 
 template <typename T>
