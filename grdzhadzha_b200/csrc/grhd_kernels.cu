@@ -1696,8 +1696,11 @@ __device__ __forceinline__ double cfl_item(const double *__restrict__ state,
             }
             return cell;
         }
+        // (the mixed path keeps the run-time background: its results stay as
+        // they are)
         GeoT<T> geo;
-        metric_T<T, false>(bg, x, y, z, geo, nullptr);
+        metric_T<T, false, sizeof(T) == sizeof(double) ? BGK : -1>(
+            bg, x, y, z, geo, nullptr);
         double gUU[6];
 #pragma unroll
         for (int q = 0; q < 6; ++q)
