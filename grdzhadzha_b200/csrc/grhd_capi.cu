@@ -1061,18 +1061,20 @@ int pipe_setup(grhd_ctx *ctx, int nchunks)
     return GRHD_OK;
 }
 
-// `bytes` of each of `rows` components (stride cs on both sides).  A pitched
-// copy of long rows saves the gaps between as many copies (a host step of
-// 161 x 143 x 127, rows of 1.5 MB: 8.0 -> 7.5 ms); with short rows (96^3, 0.6
-// MB: 2.91 against 2.98) separate copies are the faster.  So goes a stride
-// above the largest pitch that is documented for the device (2^31 - 1 bytes,
-// a box of 646^3 cells), which drivers may refuse.
+// `bytes` of each of `rows` components (stride cs on both sides) in one
+// pitched copy: it saves the gaps between as many copies.  A host step takes,
+// against separate copies, 0.31 and 0.42 ms at 16^3 (rows of 0.03 MB), 1.44
+// and 1.50 at 64^3 (0.3 MB), 2.23 and 2.19 at 80^3 (0.45 MB), 3.02 and 3.12
+// at 96^3 (0.64 MB), 6.1 and 6.7 at 128^3 (1.1 MB), 23.8 and 26.0 at 224^3
+// (4.2 MB).  A stride above the largest pitch that is documented for the
+// device (2^31 - 1 bytes, a box of 646^3 cells), which drivers may refuse,
+// takes separate copies.
 cudaError_t copy_components(const grhd_ctx *ctx, double *dst,
                             const double *src, size_t cs, size_t bytes,
                             int rows, cudaMemcpyKind kind, cudaStream_t s)
 {
     const size_t pitch = cs * sizeof(double);
-    if (bytes >= (size_t)1 << 20 && pitch <= (size_t)ctx->max_pitch)
+    if (pitch <= (size_t)ctx->max_pitch)
         return cudaMemcpy2DAsync(dst, pitch, src, pitch, bytes, rows, kind, s);
     cudaError_t e = cudaSuccess;
     for (int q = 0; q < rows && e == cudaSuccess; ++q)

@@ -1,9 +1,8 @@
-"""The copies of grhd_advance_rk4_cfl_host whose component rows are long
-(1 MB and more go as one pitched copy): a 132 x 128 x 20 box, whose chunks of
-8 planes have rows of 1.15 MB and a last one of 6 ghosted planes shorter
-ones, with an excised region eight planes and more across, so that the copies
-of all components, of the conserved ones and of those around the pressure
-take both ways.  The results equal the device step's bit for bit, and every
+"""The copies of grhd_advance_rk4_cfl_host (a chunk's components go as one
+pitched copy) with long rows: a 132 x 128 x 20 box, whose chunks of 8 planes
+have rows of 1.15 MB and a last one of 6 ghosted planes shorter ones, with an
+excised region eight planes and more across, so that all components, the
+conserved ones and those around the pressure are copied.  The results equal the device step's bit for bit, and every
 primitive that the step does not read is NaN beforehand.  The same state with
 a component stride above the largest pitch a pitched copy may have (2^31 - 1
 bytes) gives the same."""
