@@ -854,7 +854,9 @@ GRHD_HD __forceinline__ double c2p_f(double p, double D, double tD, double S2,
 }
 
 // The root solve of recover_primitive, Valencia.hpp:116-228 (bounded loops
-// throughout): the reference's bracket, start and accepted iterate.  Its
+// throughout): the reference's bracket, start, steps and acceptance, on a
+// residual that rounds differently, so that an iterate with |f| at the
+// tolerance may be accepted where the reference takes one step more.  Its
 // chain of dependent FP64 operations is what it costs, so the residuals at
 // the pressure floor and at the start, which do not depend on one another,
 // are evaluated side by side, and the residual at the bracket's upper end
@@ -972,8 +974,8 @@ GRHD_HD __forceinline__ bool c2p_finish_gUU(const Options &o, const Cons &c,
 }
 
 // The mixed path's bracketed solve: the same root solve one residual at a
-// time.  Its kernels hold three blocks per SM at 80 registers, where
-// c2p_solve's overlapped residuals spill (stage kernel: 224 -> 356 bytes).
+// time.  Its kernels that hold three blocks per SM at 80 registers spill with
+// c2p_solve's overlapped residuals (stage kernel: 224 -> 356 bytes).
 GRHD_HD __forceinline__ bool con2prim_mixed(const Options &o, const Cons &c,
                                          const double gUU[6], Prim &out,
                                          int *iters_out, double *resid_out)
@@ -1245,9 +1247,9 @@ GRHD_HD __forceinline__ double limited_slope_f64(double l, double c, double r,
 // root for W, one square root and one reciprocal for the speeds -- four
 // special functions per side where the separate formulas take eight.  The
 // face kernel is bound by issue and FP64 latency, so the operations removed
-// are time removed: with limited_slope_f64 and hlle_flux an RK4 step of the
+// are time removed: with a cheaper limiter and HLLE flux an RK4 step of the
 // 256^3 torus went from 29.8 to 24.9 ms, the 64^3 Michel step from 0.81 to
-// 0.68 ms (spill stores of the Kerr-Schild face kernel 116 -> 24 bytes).
+// 0.68 ms.
 struct FaceSide
 {
     Cons c, f;
@@ -1541,10 +1543,12 @@ GRHD_HD __forceinline__ ConsT<T> static_sources(const PrimT<T> &pr,
 // H and l with the fluid directly (ks_sources).  Sums are fma() and products
 // mul_(): every kernel that calls these gets the same bits.
 // The stage kernel was bound by the spills of those 55 values (580 MB of
-// local stores at 128^3) and by the length of the recovery's chain; with
-// this, c2p_solve and 32-bit cell indices it holds 128 registers without a
-// spill: 2.77 -> 1.55 ms per launch at 256^3 (bytes alone: 0.72), the RK4
-// step 21.0 -> 15.8 ms.
+// local stores at 128^3) and by the length of the recovery's chain.  With
+// this, c2p_solve and 32-bit cell indices it took 1.55 ms per launch at 256^3
+// instead of 2.77 at two blocks per SM (bytes alone: 0.72), and fits three
+// blocks of 80 registers (262 MB of local stores into L2 at 128^3), with which
+// and its prefetched inputs it takes 1.20.
+
 // gamma^ij S_j
 template <typename T>
 GRHD_HD __forceinline__ void ks_raise(const KsCellT<T> &k, const double S[3],

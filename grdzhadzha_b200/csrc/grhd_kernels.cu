@@ -1058,8 +1058,9 @@ __global__ void k_mdot_sum(const double *__restrict__ part, int64_t n,
 // recover_primitives_and_apply_atmosphere_from_fixed_background for one
 // cell (FixedBGFArrayBoxFiniteVolume.hpp:60-110); c is the updated
 // conserved state.  Writes prims (and reset conserved) to `out`.  With kc the
-// root solve is the Kerr-Schild cell's, the FP64 right-hand side's own: a
-// state's recovered pressures are those its right-hand side starts from.
+// root solve is the Kerr-Schild cell's, the FP64 right-hand side's own, which
+// therefore recovers the same pressures from this state; the mixed right-hand
+// side starts its own solve (con2prim_warm) from them.
 __device__ __forceinline__ void recover_cell(const Options &o, const Geo &g,
                                              const KsCell *kc, Cons c,
                                              double *out, int64_t cs,

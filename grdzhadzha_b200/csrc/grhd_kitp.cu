@@ -1,7 +1,7 @@
 // grhd_kitp.cu -- device kernels of the binary-PN disk driver's source terms
 // (alpha viscosity, point-mass sinks); see grhd_kitp.cuh.  One thread per
-// interior cell; the stencil reads go through L1 (each cell's primitives
-// are read by up to nine viscous-flux evaluations of its neighbours).
+// interior cell; the viscous fluxes of a tile and its rim are evaluated once,
+// into shared memory, from primitives read through L1.
 #include "grhd_kitp.cuh"
 
 namespace grhd {
