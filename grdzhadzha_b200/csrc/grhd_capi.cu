@@ -41,7 +41,6 @@ struct grhd_ctx
     size_t ccz4_geo_cap = 0;
     double *ccz4_stage = nullptr; // CCZ4 operator: SSPRK2 stage (GRHD)
     size_t ccz4_stage_cap = 0;
-    int max_pitch = 0;            // of a pitched copy, bytes
     double *host_state = nullptr; // device copy of a host-held state
     size_t host_state_cap = 0;
     double *prim2 = nullptr; // host-buffer step: second primitive cache
@@ -557,8 +556,6 @@ int grhd_create(const grhd_params *params, grhd_ctx **out)
     ctx->opt = make_options(*params);
     std::memset(&ctx->last_error, 0, sizeof(ctx->last_error));
     if (cudaGetDevice(&ctx->device) != cudaSuccess ||
-        cudaDeviceGetAttribute(&ctx->max_pitch, cudaDevAttrMaxPitch,
-                               ctx->device) != cudaSuccess ||
         configure_kernels() != cudaSuccess ||
         cudaMalloc((void **)&ctx->status, sizeof(DevStatus)) != cudaSuccess ||
         cudaMallocHost((void **)&ctx->status_h, sizeof(DevStatus)) !=
@@ -1066,15 +1063,15 @@ int pipe_setup(grhd_ctx *ctx, int nchunks)
 // against separate copies, 0.31 and 0.42 ms at 16^3 (rows of 0.03 MB), 1.44
 // and 1.50 at 64^3 (0.3 MB), 2.23 and 2.19 at 80^3 (0.45 MB), 3.02 and 3.12
 // at 96^3 (0.64 MB), 6.1 and 6.7 at 128^3 (1.1 MB), 23.8 and 26.0 at 224^3
-// (4.2 MB).  A stride above the largest pitch that is documented for the
-// device (2^31 - 1 bytes, a box of 646^3 cells), which drivers may refuse,
-// takes separate copies.
-cudaError_t copy_components(const grhd_ctx *ctx, double *dst,
-                            const double *src, size_t cs, size_t bytes,
-                            int rows, cudaMemcpyKind kind, cudaStream_t s)
+// (4.2 MB).  A stride above the largest pitch that CUDA documents (2^31 - 1
+// bytes, a box of 646^3 cells), which drivers may refuse, takes separate
+// copies.
+cudaError_t copy_components(double *dst, const double *src, size_t cs,
+                            size_t bytes, int rows, cudaMemcpyKind kind,
+                            cudaStream_t s)
 {
     const size_t pitch = cs * sizeof(double);
-    if (pitch <= (size_t)ctx->max_pitch)
+    if (pitch <= (size_t)INT32_MAX)
         return cudaMemcpy2DAsync(dst, pitch, src, pitch, bytes, rows, kind, s);
     cudaError_t e = cudaSuccess;
     for (int q = 0; q < rows && e == cudaSuccess; ++q)
@@ -1126,7 +1123,7 @@ int enqueue_rk4_host_pipelined(grhd_ctx *ctx, double *host, double *dev,
             const size_t bytes =
                 (size_t)(q1 - q0 + 1) * plane * sizeof(double);
             in += (long long)(bytes * (last - first));
-            return copy_components(ctx, dev + at, host + at, cs, bytes,
+            return copy_components(dev + at, host + at, cs, bytes,
                                    last - first, cudaMemcpyHostToDevice,
                                    ctx->h2d);
         };
@@ -1203,7 +1200,7 @@ int enqueue_rk4_host_pipelined(grhd_ctx *ctx, double *host, double *dev,
                 const size_t off = (size_t)(z.plo(j) - b.glo[2]) * plane;
                 const size_t n = (size_t)(z.phi(j) - z.plo(j) + 1) * plane;
                 GRHD_CUDA(ctx, copy_components(
-                                   ctx, host + off, dev + off, cs,
+                                   host + off, dev + off, cs,
                                    n * sizeof(double), kStateComps,
                                    cudaMemcpyDeviceToHost, ctx->d2h));
                 out += (long long)(n * sizeof(double) * kStateComps);
